@@ -101,6 +101,7 @@ __global__ void g_scan_rows_kernel(const GSplitProb* __restrict__ P, int count, 
 }
 
 constexpr int kScanKChunk = 256;  // rows of B one column-scan unit covers
+static_assert(kScanKChunk == kNormChunk, "the modular scan's chunk");
 
 __global__ void g_reset_cols_kernel(const GSplitProb* __restrict__ P, int count, int total_cols) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -153,10 +154,8 @@ __global__ void g_scan_cols_part_kernel(const GSplitProb* __restrict__ P, int co
   const int w = u - p.cunit_start;
   const int64_t col = w % p.n;
   const int chunk = w / p.n;
-  const int k0 = chunk * kScanKChunk, k1 = min(p.k, k0 + kScanKChunk);
-  NormAcc acc;
   bool nf = false;
-  norm_col_chunk(p.B, p.ldb, col, k0, k1, acc, nf);
+  const NormAcc acc = norm_col_chunk(p.B, p.ldb, col, chunk * kNormChunk, p.k, nf);
   p.pe[(int64_t)chunk * p.n + col] = acc.e;
   p.ps[(int64_t)chunk * p.n + col] = acc.s;
   if (nf) record_error(status, PHPC_ERR_NONFINITE);
@@ -169,14 +168,7 @@ __global__ void g_scan_cols_merge_kernel(const GSplitProb* __restrict__ P, int c
   if (c >= total_cols) return;
   const GSplitProb& p = P[locate_warp(P, count, c, [](const GSplitProb& q) { return q.col_start; })];
   const int64_t col = c - p.col_start;
-  const int chunks = (p.k + kScanKChunk - 1) / kScanKChunk;
-  NormAcc acc;
-  for (int ch = 0; ch < chunks; ++ch) {
-    NormAcc q;
-    q.e = p.pe[(int64_t)ch * p.n + col];
-    q.s = p.ps[(int64_t)ch * p.n + col];
-    norm_merge(acc, q);
-  }
+  const NormAcc acc = norm_merge_chunks(p.pe, p.ps, p.n, col, (p.k + kNormChunk - 1) / kNormChunk);
   p.eb[col] = acc.e;
   p.bb[col] = grid_bits(acc.s, p.k, T.logT);
 }
@@ -254,8 +246,9 @@ __global__ void __launch_bounds__(256, 4) g_residue_cols_kernel(const GSplitProb
   const int lb = b - p.rblock_start;
   const int nblk_j = (p.n + kColBlockJ - 1) / kColBlockJ;
   __shared__ double tile[kColBlockK][kColBlockJ];
-  residue_col_block<NMOD>(p.B, p.ldb, p.k, p.n, (int64_t)(lb % nblk_j) * kColBlockJ, (int64_t)(lb / nblk_j) * kColBlockK,
-                          p.eb, p.bb, T, p.pb, p.ldp, (int64_t)p.n * p.ldp, tile);
+  const int64_t j0 = (int64_t)(lb % nblk_j) * kColBlockJ, col = min(j0 + (threadIdx.x >> 3), (int64_t)p.n - 1);
+  residue_col_block<NMOD>(p.B, p.ldb, p.k, p.n, j0, (int64_t)(lb / nblk_j) * kColBlockK, p.eb[col], p.bb[col], T,
+                          p.pb, p.ldp, (int64_t)p.n * p.ldp, tile);
 }
 
 // CRT units: 32 groups of kCrtCols consecutive columns of one row (a

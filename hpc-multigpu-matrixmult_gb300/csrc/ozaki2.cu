@@ -56,39 +56,34 @@ __global__ void scan_rows_grid_kernel(const double* __restrict__ A, int64_t lda,
   if (__any_sync(0xffffffffu, nf) && (threadIdx.x & 31) == 0) record_error(status, PHPC_ERR_NONFINITE);
 }
 
-constexpr int kGridKChunk = 256;  // rows of B one column-scan thread covers
-
-// Column scan, part 1: thread (column j, chunk c) keeps the exponent and the
-// scaled sum of squares of B[256c .. 256c + 255][j] in pe / ps [chunk][n].
-__global__ void scan_cols_part_kernel(const double* __restrict__ B, int64_t ldb, int K, int N, int64_t ldpart,
-                                      int* __restrict__ pe, float* __restrict__ ps, int* status) {
-  const int64_t col = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (col >= N) return;
-  const int k0 = blockIdx.y * kGridKChunk, k1 = min(K, k0 + kGridKChunk);
+// Column scan, part 1: block (strip of 32 columns, chunk of 256 rows); warp w
+// sums rows 32 w .. + 31 of the chunk, and warp 0 merges the eight slices in
+// order into pe / ps [chunk][n]. A column's chain is 32 FMAs with 16 loads in
+// flight, and even N = 256 has 8 blocks; one thread per column and 256 rows
+// took 53-59 us at every size up to N = 4096 (the chain's latency) and 410 us
+// at N = 16384, against 4 us at N = 256, 5.5 at 1024, 22 at 4096 and 292 at
+// 16384 (7.3 TB/s) for this.
+__global__ void __launch_bounds__(256) scan_cols_part_kernel(const double* __restrict__ B, int64_t ldb, int K, int N,
+                                                             int64_t ldpart, int* __restrict__ pe,
+                                                             float* __restrict__ ps, int* status) {
+  __shared__ int se[8][32];
+  __shared__ float ss[8][32];
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  const int64_t col = (int64_t)blockIdx.x * 32 + l;
+  const int k0 = blockIdx.y * kNormChunk + w * kNormSlice;
   NormAcc acc;
   bool nf = false;
-  norm_col_chunk(B, ldb, col, k0, k1, acc, nf);
+  if (col < N && k0 < K) norm_col_slice(B, ldb, col, k0, K, acc, nf);
+  se[w][l] = acc.e;
+  ss[w][l] = acc.s;
+  if (nf) record_error(status, PHPC_ERR_NONFINITE);
+  __syncthreads();
+  if (w != 0 || col >= N) return;
+  acc = NormAcc{};
+#pragma unroll
+  for (int u = 0; u < 8; ++u) norm_merge(acc, NormAcc{se[u][l], ss[u][l]});
   pe[blockIdx.y * ldpart + col] = acc.e;
   ps[blockIdx.y * ldpart + col] = acc.s;
-  if (nf) record_error(status, PHPC_ERR_NONFINITE);
-}
-
-// Column scan, part 2: eb[j] and bb[j] from the chunks, merged in order.
-__global__ void scan_cols_merge_kernel(int K, int N, int64_t ldpart, const int* __restrict__ pe,
-                                       const float* __restrict__ ps, int* __restrict__ eb, int* __restrict__ bb,
-                                       float logT) {
-  const int64_t col = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (col >= N) return;
-  const int chunks = (K + kGridKChunk - 1) / kGridKChunk;
-  NormAcc acc;
-  for (int c = 0; c < chunks; ++c) {
-    NormAcc p;
-    p.e = pe[c * ldpart + col];
-    p.s = ps[c * ldpart + col];
-    norm_merge(acc, p);
-  }
-  eb[col] = acc.e;
-  bb[col] = grid_bits(acc.s, K, logT);
 }
 
 // A residue planes [n][M][ldp]: blockIdx.x = row, each thread 8 consecutive k.
@@ -103,17 +98,65 @@ __global__ void residue_rows_kernel(const double* __restrict__ A, int64_t lda, i
   residue_row_piece<NMOD>(A + row * lda, K, ea[row], ba[row], T, planes + row * ldp, plane_stride, k0);
 }
 
+// Column scan, part 2: a block merges the chunks of 32 columns, warp p those
+// numbered p, p + 8, ..., into eb[j] and bb[j].
+__global__ void __launch_bounds__(256) scan_cols_merge_kernel(int K, int N, int64_t ldpart,
+                                                              const int* __restrict__ pe,
+                                                              const float* __restrict__ ps, int* __restrict__ eb,
+                                                              int* __restrict__ bb, float logT) {
+  __shared__ int se[8][32];
+  __shared__ float ss[8][32];
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  const int64_t col = (int64_t)blockIdx.x * 32 + l;
+  const int chunks = (K + kNormChunk - 1) / kNormChunk;
+  NormAcc acc = norm_merge_strided(pe, ps, ldpart, col, col < N ? chunks : 0, w);
+  se[w][l] = acc.e;
+  ss[w][l] = acc.s;
+  __syncthreads();
+  if (w != 0 || col >= N) return;
+  NormAcc q[8];
+#pragma unroll
+  for (int p = 0; p < 8; ++p) q[p] = NormAcc{se[p][l], ss[p][l]};
+  acc = norm_merge_tree(q);
+  eb[col] = acc.e;
+  bb[col] = grid_bits(acc.s, K, logT);
+}
+
+// Up to this many chunks (K <= 1024) the column split merges them itself: a
+// merge kernel is 3-4 us of a small call, the merge in every block of the
+// split 0.6 us of 11 at N = 1024 (but 22 us of 120 at N = 4096, 0.9 ms of
+// 2.4 at 16384).
+constexpr int kMergeInSplit = 4;
+
 // B residue planes, transposed ([n][N][ldp]): one kColBlockK x kColBlockJ
-// block per 256-thread CTA (residue.cuh).
+// block per 256-thread CTA (residue.cuh). With pe the eight threads of a
+// column merge its chunks into the exponent and grid width, and the first row
+// of blocks stores them in eb / bb for the CRT; without, eb / bb are there.
 template <int NMOD>
 __global__ void __launch_bounds__(256) residue_cols_kernel(const double* __restrict__ B, int64_t ldb, int K, int N,
-                                                           const int* __restrict__ eb, const int* __restrict__ bb,
+                                                           int64_t ldpart, const int* __restrict__ pe,
+                                                           const float* __restrict__ ps, int* eb, int* bb,
                                                            const __grid_constant__ ModTable T,
                                                            uint16_t* __restrict__ planes, int64_t ldp,
                                                            int64_t plane_stride) {
   __shared__ double tile[kColBlockK][kColBlockJ];
-  residue_col_block<NMOD>(B, ldb, K, N, (int64_t)blockIdx.x * kColBlockJ, (int64_t)blockIdx.y * kColBlockK, eb, bb,
-                          T, planes, ldp, plane_stride, tile);
+  const int64_t j0 = (int64_t)blockIdx.x * kColBlockJ, col = j0 + (threadIdx.x >> 3);
+  int e, bits;
+  if (pe) {
+    const int chunks = (K + kNormChunk - 1) / kNormChunk;
+    const NormAcc acc = norm_merge_chunks8(pe, ps, ldpart, col, col < N ? chunks : 0, threadIdx.x & 7);
+    e = acc.e;
+    bits = grid_bits(acc.s, K, T.logT);
+    if (blockIdx.y == 0 && col < N && (threadIdx.x & 7) == 0) {
+      eb[col] = e;
+      bb[col] = bits;
+    }
+  } else {
+    e = col < N ? eb[col] : 0;
+    bits = col < N ? bb[col] : 0;
+  }
+  residue_col_block<NMOD>(B, ldb, K, N, j0, (int64_t)blockIdx.y * kColBlockK, e, bits, T, planes, ldp, plane_stride,
+                          tile);
 }
 
 // C[i][j] += C_int * 2^(ea[i] - ba[i] + eb[j] - bb[j]), C_int recovered from the residues.
@@ -144,7 +187,7 @@ Ozaki2Layout ozaki2_layout(int m, int k, int n, int nmod) {
   L.ldp = ((int64_t)k + 7) / 8 * 8;
   L.ldr = ((int64_t)n + 15) / 16 * 16;
   L.ldpart = n;
-  const size_t chunks = (static_cast<size_t>(k) + kGridKChunk - 1) / kGridKChunk;
+  const size_t chunks = (static_cast<size_t>(k) + kNormChunk - 1) / kNormChunk;
   L.off_ea = 0;
   L.off_eb = align256(sizeof(int) * (size_t)m);
   L.off_ba = align256(L.off_eb + sizeof(int) * (size_t)n);
@@ -227,16 +270,20 @@ int ozaki2_prepare_b_cols(int m, int k, int n, int c0, int cols, const double* d
   if (c0 < 0 || cols <= 0 || c0 + cols > n) return PHPC_ERR_ARG;
   const ModTable T = make_table(nmod, k);
   const double* b = dB + c0;
+  scan_cols_part_kernel<<<dim3(ceil_div(cols, 32), ceil_div(k, kNormChunk)), 256, 0, stream>>>(
+      b, ldb, k, cols, L.ldpart, V.pe + c0, V.ps + c0, device_status_ptr());
   int* eb = V.eb + c0;
   int* bb = V.bb + c0;
-  scan_cols_part_kernel<<<dim3(ceil_div(cols, 256), ceil_div(k, kGridKChunk)), 256, 0, stream>>>(
-      b, ldb, k, cols, L.ldpart, V.pe + c0, V.ps + c0, device_status_ptr());
-  scan_cols_merge_kernel<<<ceil_div(cols, 256), 256, 0, stream>>>(k, cols, L.ldpart, V.pe + c0, V.ps + c0, eb, bb,
-                                                                 T.logT);
+  const bool merge = ceil_div(k, kNormChunk) > kMergeInSplit;
+  if (merge)
+    scan_cols_merge_kernel<<<ceil_div(cols, 32), 256, 0, stream>>>(k, cols, L.ldpart, V.pe + c0, V.ps + c0, eb, bb,
+                                                                  T.logT);
+  const int* pe = merge ? nullptr : V.pe + c0;
   with_crt_moduli(T.n, [&](auto nm) {
     residue_cols_kernel<decltype(nm)::value>
         <<<dim3(ceil_div(cols, kColBlockJ), ceil_div(L.ldp, kColBlockK)), 256, 0, stream>>>(
-            b, ldb, k, cols, eb, bb, T, V.pb + (int64_t)c0 * L.ldp, L.ldp, (int64_t)n * L.ldp);
+            b, ldb, k, cols, L.ldpart, pe, V.ps + c0, eb, bb, T, V.pb + (int64_t)c0 * L.ldp, L.ldp,
+            (int64_t)n * L.ldp);
   });
   PHPC_CUDA_TRY(cudaGetLastError());
   return PHPC_OK;

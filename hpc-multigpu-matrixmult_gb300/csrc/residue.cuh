@@ -188,12 +188,47 @@ __device__ __forceinline__ void norm_add(NormAcc& a, double x, bool& nonfinite) 
   }
 }
 
+// 2^d for d <= 0 as a float, 0 below the normal range (the larger of two
+// merged sums is at least 1/4, so what that drops is below its rounding).
+__device__ __forceinline__ float pow2_down(int d) {
+  return d < -126 ? 0.0f : __uint_as_float(static_cast<uint32_t>(127 + d) << 23);
+}
+
+// norm_add of N values at once, the same sum: the exponent is raised to the
+// largest of the batch first (scaling by powers of two commutes with the
+// rounding of the sum), so the chain from element to element is one FMA. The
+// scaled value is scaled_abs_up's, cut from the two words of the double by a
+// funnel shift. Batches whose largest exponent is below 2^-862 (subnormal
+// values could count), or that hold an inf/NaN, go element by element.
+template <int N>
+__device__ __forceinline__ void norm_add_batch(NormAcc& a, const double (&x)[N], bool& nonfinite) {
+  constexpr uint32_t kAbs = 0x7FFFFFFFu, kTiny = 160u << 20, kInf = 0x7FFu << 20;
+  uint32_t mx = 0;
+#pragma unroll
+  for (int u = 0; u < N; ++u) mx = max(mx, static_cast<uint32_t>(__double2hiint(x[u])) & kAbs);
+  if (mx < kTiny || mx >= kInf) {
+#pragma unroll
+    for (int u = 0; u < N; ++u) norm_add(a, x[u], nonfinite);
+    return;
+  }
+  const int e = max(a.e, static_cast<int>(mx >> 20) - 1022);
+  a.s *= pow2_down(2 * max(a.e - e, -100));
+  a.e = e;
+  if (e >= kExpNonFinite) return;  // an earlier inf/NaN
+  const int rebias = (e + 896) << 20;  // biased double exponent E -> float exponent E - 896 - e of |x| 2^-e
+#pragma unroll
+  for (int u = 0; u < N; ++u) {
+    const int hi = static_cast<int>(static_cast<uint32_t>(__double2hiint(x[u])) & kAbs) - rebias;
+    const uint32_t f = __funnelshift_l(static_cast<uint32_t>(__double2loint(x[u])), static_cast<uint32_t>(hi), 3) + 1u;
+    const float v = hi < (1 << 20) ? 0.0f : __uint_as_float(f);  // below 2^-126: its square is 0
+    a.s = fmaf(v, v, a.s);
+  }
+}
+
 __device__ __forceinline__ void norm_merge(NormAcc& a, const NormAcc& b) {
   const int e = max(a.e, b.e);
-  const float sa = a.e > kExpZero ? ldexpf(a.s, 2 * (a.e - e)) : 0.0f;
-  const float sb = b.e > kExpZero ? ldexpf(b.s, 2 * (b.e - e)) : 0.0f;
+  a.s = a.s * pow2_down(2 * max(a.e - e, -100)) + b.s * pow2_down(2 * max(b.e - e, -100));
   a.e = e;
-  a.s = sa + sb;
 }
 
 // Merge over the 32 lanes of a warp (every lane gets the result).
@@ -209,34 +244,94 @@ __device__ __forceinline__ NormAcc norm_warp(NormAcc a) {
 }
 
 // One lane's share of a row's scan: elements lane, lane + 32, ... in that
-// order, four loads issued before they are accumulated. (Eight measured
-// 3 % faster on 16384-element rows and 20 % slower on the batch's short
-// rows.)
+// order, eight loads in flight.
 __device__ __forceinline__ void norm_row_lane(const double* __restrict__ a, int K, int lane, NormAcc& acc,
                                               bool& nonfinite) {
-  int k = lane;
-  for (; k + 96 < K; k += 128) {
-    const double x0 = a[k], x1 = a[k + 32], x2 = a[k + 64], x3 = a[k + 96];
-    norm_add(acc, x0, nonfinite);
-    norm_add(acc, x1, nonfinite);
-    norm_add(acc, x2, nonfinite);
-    norm_add(acc, x3, nonfinite);
-  }
-  for (; k < K; k += 32) norm_add(acc, a[k], nonfinite);
-}
-
-// Rows k0 .. k1 - 1 of column col of B, in order, eight loads at a time.
-__device__ __forceinline__ void norm_col_chunk(const double* __restrict__ B, int64_t ldb, int64_t col, int k0, int k1,
-                                               NormAcc& acc, bool& nonfinite) {
-  int k = k0;
-  for (; k + 7 < k1; k += 8) {
+  for (int k = lane; k < K; k += 256) {
     double x[8];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) x[u] = B[(int64_t)(k + u) * ldb + col];
-#pragma unroll
-    for (int u = 0; u < 8; ++u) norm_add(acc, x[u], nonfinite);
+    for (int u = 0; u < 8; ++u) x[u] = k + 32 * u < K ? a[k + 32 * u] : 0.0;
+    norm_add_batch(acc, x, nonfinite);
   }
-  for (; k < k1; ++k) norm_add(acc, B[(int64_t)k * ldb + col], nonfinite);
+}
+
+// The column scan's order, the same for the single and the grouped call: a
+// chunk is 256 rows, a slice 32 of them; a slice is summed row by row, a
+// chunk's eight slices are merged in order, and a column's chunks by
+// norm_merge_chunks.
+constexpr int kNormChunk = 256, kNormSlice = 32;
+
+// Slice [k0, min(k0 + 32, K)) of column col of B, 16 loads in flight.
+__device__ __forceinline__ void norm_col_slice(const double* __restrict__ B, int64_t ldb, int64_t col, int k0, int K,
+                                               NormAcc& acc, bool& nonfinite) {
+  const double* b = B + k0 * ldb + col;
+#pragma unroll
+  for (int h = 0; h < kNormSlice; h += 16) {
+    double x[16];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) x[u] = k0 + h + u < K ? b[(h + u) * ldb] : 0.0;
+    norm_add_batch(acc, x, nonfinite);
+  }
+}
+
+// One chunk of column col by one thread.
+__device__ __forceinline__ NormAcc norm_col_chunk(const double* __restrict__ B, int64_t ldb, int64_t col, int k0,
+                                                  int K, bool& nonfinite) {
+  NormAcc acc;
+  for (int k = k0; k < min(k0 + kNormChunk, K); k += kNormSlice) {
+    NormAcc s;
+    norm_col_slice(B, ldb, col, k, K, s, nonfinite);
+    norm_merge(acc, s);
+  }
+  return acc;
+}
+
+// Chunks p, p + 8, ... of a column's partials pe / ps [chunk][ld], in order.
+__device__ __forceinline__ NormAcc norm_merge_strided(const int* __restrict__ pe, const float* __restrict__ ps,
+                                                      int64_t ld, int64_t col, int chunks, int p) {
+  NormAcc acc;
+#pragma unroll 4
+  for (int c = p; c < chunks; c += 8) {
+    NormAcc q;
+    q.e = pe[c * ld + col];
+    q.s = ps[c * ld + col];
+    norm_merge(acc, q);
+  }
+  return acc;
+}
+
+// All chunks of a column: eight interleaved merges, combined pairwise. By
+// eight consecutive lanes (p = lane % 8; every lane gets the result, all 32
+// lanes of the warp must call it) ...
+__device__ __forceinline__ NormAcc norm_merge_chunks8(const int* __restrict__ pe, const float* __restrict__ ps,
+                                                      int64_t ld, int64_t col, int chunks, int p) {
+  NormAcc acc = norm_merge_strided(pe, ps, ld, col, chunks, p);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) {
+    NormAcc b;
+    b.e = __shfl_xor_sync(0xffffffffu, acc.e, o);
+    b.s = __shfl_xor_sync(0xffffffffu, acc.s, o);
+    norm_merge(acc, b);
+  }
+  return acc;
+}
+
+// The same combination of the eight merges q by one thread ...
+__device__ __forceinline__ NormAcc norm_merge_tree(NormAcc (&q)[8]) {
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+    for (int p = 0; p < o; ++p) norm_merge(q[p], q[p + o]);
+  return q[0];
+}
+
+// ... and all of a column's chunks by one thread.
+__device__ __forceinline__ NormAcc norm_merge_chunks(const int* __restrict__ pe, const float* __restrict__ ps,
+                                                     int64_t ld, int64_t col, int chunks) {
+  NormAcc q[8];
+#pragma unroll
+  for (int p = 0; p < 8; ++p) q[p] = norm_merge_strided(pe, ps, ld, col, chunks, p);
+  return norm_merge_tree(q);
 }
 
 // Grid width of a row/column with scaled sum of squares s over K elements.
@@ -361,13 +456,13 @@ __device__ __forceinline__ void residue_row_piece(const double* __restrict__ a, 
 // shared memory (tile, 64 x 32 doubles): warp w reads rows w, w + 8, ... as
 // whole 256-byte row segments; then thread t takes column j0 + t / 8 and
 // rows 8 (t % 8) .. + 7, so that the 8 threads of one column write one
-// contiguous 128-byte run of each plane row. Element (k, j) sits at
+// contiguous 128-byte run of each plane row; e and bits are that column's
+// exponent and grid width. Element (k, j) sits at
 // tile[k][j ^ 4 ((k / 8) % 4)], which keeps both the row writes and the
 // column reads at two shared-memory wavefronts per warp access.
 template <int NMOD>
 __device__ __forceinline__ void residue_col_block(const double* __restrict__ B, int64_t ldb, int K, int N,
-                                                  int64_t j0, int64_t k0, const int* __restrict__ eb,
-                                                  const int* __restrict__ bb, const ModTable& T,
+                                                  int64_t j0, int64_t k0, int e, int bits, const ModTable& T,
                                                   uint16_t* __restrict__ planes, int64_t ldp, int64_t plane_stride,
                                                   double (&tile)[64][32]) {
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
@@ -385,7 +480,7 @@ __device__ __forceinline__ void residue_col_block(const double* __restrict__ B, 
 #pragma unroll
   for (int u = 0; u < 8; ++u) v[u] = tile[8 * p + u][jj ^ (4 * (p & 3))];
   float2 P[4][kLimbs];
-  limb_pairs(v, eb[col], bb[col], P);
+  limb_pairs(v, e, bits, P);
   store_residues8<NMOD, false>(P, T, planes + col * ldp + kp, plane_stride);
 }
 
