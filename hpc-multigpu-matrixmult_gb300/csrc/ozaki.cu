@@ -135,29 +135,26 @@ int launch_tc_slice_gemm(const void* planesA, const void* planesB, int nplanesA,
   a.ldr = ldr;
   a.rplane = rplane;
   if (MODE == kResidue) {
-    // split the moduli into separate work units, moduli outer, when the
-    // tiles fill at least one wave of SMs: consecutive waves then work on the
-    // same modulus and share its planes in L2, and a ragged last wave is
-    // spread over 13x more units (single CTAs, N = 4096: 14 % faster, DRAM
-    // traffic 2.1x -> 1.06x the algorithmic bytes; N = 8192: 3 %; N = 16384:
-    // 1-2 %, DRAM reads 145 -> 112 GB). Below one wave of tiles it measured
-    // 2-7 % slower. A CTA pair's tile is 256 rows high and a wave has half as
-    // many of them.
-    int split = opt.split_pairs;
-    if (const char* env = getenv("PHPC_SPLIT_MODULI")) split = atoi(env) != 0 ? 1 : 0;
-    const int64_t tiles = cluster == 1 ? (int64_t)a.tm * a.tn : (int64_t)((a.tm + 1) / 2) * a.tn;
-    if (split < 0) split = tiles * cluster >= dev->sm_count ? 1 : 0;
-    a.split_pairs = split;
+    // One work unit per (tile, modulus), moduli outer: consecutive waves work
+    // on the same modulus and share its planes in L2, a ragged last wave is
+    // spread over 13x more units, and a problem of few tiles still reaches
+    // every SM (the grid is one CTA per unit up to the SM count). Against one
+    // unit per tile (PHPC_SPLIT_MODULI = 0), BN = 256: N = 512 54 -> 13 us,
+    // 1024 92 -> 28, 2048 168 -> 148, 4096 1282 -> 1046; no size measured
+    // (256 to 16384, short and long K) is slower.
+    const char* split = getenv("PHPC_SPLIT_MODULI");
+    a.split_pairs = split ? (atoi(split) != 0 ? 1 : 0) : 1;
     // odd rounds of units walk K backwards (PHPC_K_SERPENTINE = 0 turns it off)
     const char* serp = getenv("PHPC_K_SERPENTINE");
     a.k_serpentine = serp ? (atoi(serp) != 0 ? 1 : 0) : 1;
   }
+  const int64_t units =
+      (cluster == 1 ? (int64_t)a.tm * a.tn : (int64_t)((a.tm + 1) / 2) * a.tn) * (a.split_pairs ? pairs.n : 1);
   if (cluster == 1) {
     auto kern = tc_slice_gemm_kernel<BN, MODE>;
     if (!tc_regs_ok(reinterpret_cast<const void*>(kern))) return PHPC_ERR_UNSUPPORTED;
     PHPC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::kSmem));
-    const int ntiles = a.tm * a.tn;
-    const int grid = std::min(ntiles, dev->sm_count);
+    const int grid = static_cast<int>(std::min<int64_t>(units, dev->sm_count));
     kern<<<grid, kTcThreads, Cfg::kSmem, stream>>>(tmA, tmB, pairs, a, TcGroupTable{});
     PHPC_CUDA_TRY(cudaGetLastError());
     return PHPC_OK;
@@ -178,12 +175,11 @@ int launch_tc_slice_gemm(const void* planesA, const void* planesB, int nplanesA,
   cfg.stream = stream;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  const int npairs = ((a.tm + 1) / 2) * a.tn;
-  cfg.gridDim = dim3(2 * std::min(npairs, dev->sm_count / 2), 1, 1);
+  cfg.gridDim = dim3(2 * static_cast<unsigned>(std::min<int64_t>(units, dev->sm_count / 2)), 1, 1);
   int max_clusters = 0;
   PHPC_CUDA_TRY(cudaOccupancyMaxActiveClusters(&max_clusters, kern, &cfg));
   if (max_clusters < 1) return PHPC_ERR_UNSUPPORTED;
-  cfg.gridDim = dim3(2 * std::min(npairs, max_clusters), 1, 1);
+  cfg.gridDim = dim3(2 * static_cast<unsigned>(std::min<int64_t>(units, max_clusters)), 1, 1);
   PHPC_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, tmA, tmB, pairs, a, TcGroupTable{}));
   return PHPC_OK;
 }
