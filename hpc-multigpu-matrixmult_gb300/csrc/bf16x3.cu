@@ -40,7 +40,7 @@ __global__ void split3_rows_kernel(const float* __restrict__ A, int64_t lda, int
                                    uint16_t* __restrict__ planes, int64_t ldp, int64_t plane_stride) {
   const int64_t row = blockIdx.x;
   const int64_t k0 = ((int64_t)blockIdx.y * blockDim.x + threadIdx.x) * 8;
-  if (row >= M || k0 >= ldp) return;
+  if (row >= M || k0 >= K) return;
   const float* a = A + row * lda;
   uint32_t w[3][4];
 #pragma unroll
@@ -77,7 +77,7 @@ __global__ void __launch_bounds__(256) split3_cols_kernel(const float* __restric
   __syncthreads();
   const int wj = threadIdx.x >> 2, q = threadIdx.x & 3;
   const int64_t gj = j0 + wj, gk = k0 + 8 * q;
-  if (gj >= N || gk >= ldp) return;
+  if (gj >= N || gk >= K) return;
 #pragma unroll
   for (int p = 0; p < 3; ++p)
     *reinterpret_cast<uint4*>(planes + p * plane_stride + gj * ldp + gk) =
@@ -171,9 +171,9 @@ struct Bf16x3Layout {
   size_t off_pa, off_pb, total;
 };
 
-Bf16x3Layout bf16x3_layout(int m, int k, int n) {
+Bf16x3Layout bf16x3_layout(int m, int k, int n, bool padded = true) {
   Bf16x3Layout L;
-  L.ldp = ((int64_t)k + 7) / 8 * 8;
+  L.ldp = plane_ld(k, padded);
   L.off_pa = 0;
   L.off_pb = align256((size_t)3 * m * L.ldp * 2);
   L.total = align256(L.off_pb + (size_t)3 * n * L.ldp * 2);
@@ -214,7 +214,8 @@ extern "C" int phpc_sgemm_bf16x3_dev(int m, int k, int n, const float* dA, int64
     rc = PHPC_ERR_ARG;
   } else {
     const DeviceInfo* dev = current_device();
-    const Bf16x3Layout L = bf16x3_layout(m, k, n);
+    Bf16x3Layout L = bf16x3_layout(m, k, n);
+    if (workspace_bytes < L.total) L = bf16x3_layout(m, k, n, false);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (!dev) {
       rc = PHPC_ERR_CUDA;
@@ -225,7 +226,7 @@ extern "C" int phpc_sgemm_bf16x3_dev(int m, int k, int n, const float* dA, int64
     } else {
       uint16_t* pa = reinterpret_cast<uint16_t*>(static_cast<uint8_t*>(workspace) + L.off_pa);
       uint16_t* pb = reinterpret_cast<uint16_t*>(static_cast<uint8_t*>(workspace) + L.off_pb);
-      split3_rows_kernel<<<dim3(m, ceil_div(L.ldp / 8, 128)), 128, 0, st>>>(dA, lda, m, k, pa, L.ldp,
+      split3_rows_kernel<<<dim3(m, ceil_div(k, 8 * 128)), 128, 0, st>>>(dA, lda, m, k, pa, L.ldp,
                                                                             (int64_t)m * L.ldp);
       split3_cols_kernel<<<dim3(ceil_div(n, 64), ceil_div(k, 32)), 256, 0, st>>>(dB, ldb, k, n, pb, L.ldp,
                                                                                  (int64_t)n * L.ldp);

@@ -183,7 +183,7 @@ struct RowPiece {
 
 __device__ __forceinline__ RowPiece row_piece(const GSplitProb* __restrict__ P, int count, int t) {
   const GSplitProb& p = P[locate_warp(P, count, t, [](const GSplitProb& q) { return q.piece_start; })];
-  const int per_row = static_cast<int>(p.ldp >> 3);
+  const int per_row = (p.k + 7) >> 3;
   const int local = t - p.piece_start;
   return RowPiece{&p, local / per_row, static_cast<int64_t>(local % per_row) * 8};
 }
@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(kResRowBlock, 4) g_residue_rows_kernel(const G
   int pi = first[blockIdx.x];
   while (pi + 1 < count && P[pi + 1].piece_start <= t) ++pi;
   const GSplitProb& p = P[pi];
-  const int per_row = static_cast<int>(p.ldp >> 3);
+  const int per_row = (p.k + 7) >> 3;
   const int local = t - p.piece_start;
   const int64_t row = local / per_row, k0 = static_cast<int64_t>(local % per_row) * 8;
   residue_row_piece<NMOD>(p.A + row * p.lda, p.k, p.ea[row], p.ba[row], T, p.pa + row * p.ldp, (int64_t)p.m * p.ldp,
@@ -300,10 +300,10 @@ struct ProbLayout {
 };
 
 // planes = slices (digit scheme) or moduli (modular scheme, which adds the
-// residue planes R).
-ProbLayout prob_layout(const phpc_gemm_problem& q, int planes, bool modular) {
+// residue planes R); padded: the modular planes' row stride (plane_ld).
+ProbLayout prob_layout(const phpc_gemm_problem& q, int planes, bool modular, bool padded) {
   ProbLayout L;
-  L.ldp = ((int64_t)q.k + 7) / 8 * 8;
+  L.ldp = plane_ld(q.k, modular && padded);
   L.ldr = ((int64_t)q.n + 15) / 16 * 16;
   const size_t chunks = modular ? (static_cast<size_t>(q.k) + kScanKChunk - 1) / kScanKChunk : 0;
   L.ea = 0;
@@ -515,11 +515,12 @@ int run_grouped(const phpc_grouped_plan* pl, cudaStream_t stream) {
   return rc;
 }
 
-size_t grouped_workspace_bytes(const phpc_gemm_problem* problems, int count, int planes, bool modular) {
+size_t grouped_workspace_bytes(const phpc_gemm_problem* problems, int count, int planes, bool modular,
+                               bool padded = true) {
   size_t total = table_layout(count, max_tiles(problems, count), lookup_sizes(problems, count, modular)).end;
   for (int i = 0; i < count; ++i) {
     if (!valid_problem(problems[i])) return 0;
-    total += prob_layout(problems[i], planes, modular).end;
+    total += prob_layout(problems[i], planes, modular, padded).end;
   }
   return total;
 }
@@ -534,7 +535,8 @@ int grouped_plan_create(phpc_grouped_plan** out, const phpc_gemm_problem* proble
   const DeviceInfo* dev = current_device();
   if (!dev) return PHPC_ERR_CUDA;
   if (dev->cc_major != 10 || dev->cc_minor != 3) return PHPC_ERR_UNSUPPORTED;
-  const size_t need = grouped_workspace_bytes(problems, count, planes, modular);
+  const bool padded = workspace_bytes >= grouped_workspace_bytes(problems, count, planes, modular);
+  const size_t need = grouped_workspace_bytes(problems, count, planes, modular, padded);
   if (!workspace || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 255))
     return PHPC_ERR_WORKSPACE;
   for (int i = 0; i < count; ++i)
@@ -566,7 +568,7 @@ int grouped_plan_create(phpc_grouped_plan** out, const phpc_gemm_problem* proble
   int64_t pieces = 0, cunits = 0, crt_units = 0;
   for (int i = 0; i < count && rc == PHPC_OK; ++i) {
     const phpc_gemm_problem& q = problems[i];
-    const ProbLayout L = prob_layout(q, planes, modular);
+    const ProbLayout L = prob_layout(q, planes, modular, padded);
     uint8_t* pb = base + off;
     GSplitProb& g = hs[i];
     g = GSplitProb{};

@@ -94,7 +94,7 @@ __global__ void residue_rows_kernel(const double* __restrict__ A, int64_t lda, i
                                     int64_t plane_stride) {
   const int64_t row = blockIdx.x;
   const int64_t k0 = ((int64_t)blockIdx.y * blockDim.x + threadIdx.x) * 8;
-  if (row >= M || k0 >= ldp) return;
+  if (row >= M || k0 >= K) return;
   residue_row_piece<NMOD>(A + row * lda, K, ea[row], ba[row], T, planes + row * ldp, plane_stride, k0);
 }
 
@@ -182,9 +182,9 @@ struct Ozaki2Layout {
 
 // Workspace: ea[m], eb[n], ba[m], bb[n], the column scan's chunk partials
 // pe / ps [ceil(k / 256)][n], A planes, B planes, residues.
-Ozaki2Layout ozaki2_layout(int m, int k, int n, int nmod) {
+Ozaki2Layout ozaki2_layout(int m, int k, int n, int nmod, bool padded = true) {
   Ozaki2Layout L;
-  L.ldp = ((int64_t)k + 7) / 8 * 8;
+  L.ldp = plane_ld(k, padded);
   L.ldr = ((int64_t)n + 15) / 16 * 16;
   L.ldpart = n;
   const size_t chunks = (static_cast<size_t>(k) + kNormChunk - 1) / kNormChunk;
@@ -218,6 +218,7 @@ int ozaki2_views(int m, int k, int n, int nmod, const void* ws, size_t ws_bytes,
   if (!dev) return PHPC_ERR_CUDA;
   if (dev->cc_major != 10 || dev->cc_minor != 3) return PHPC_ERR_UNSUPPORTED;
   L = ozaki2_layout(m, k, n, nmod);
+  if (ws_bytes < L.total) L = ozaki2_layout(m, k, n, nmod, false);
   if (!ws || ws_bytes < L.total || !aligned16(ws)) return PHPC_ERR_WORKSPACE;
   uint8_t* base = static_cast<uint8_t*>(const_cast<void*>(ws));
   V.ea = reinterpret_cast<int*>(base + L.off_ea);
@@ -252,7 +253,7 @@ int ozaki2_prepare_a_rows(int m, int r0, int rows, int k, int n, const double* d
   scan_rows_grid_kernel<<<ceil_div(rows, 8), 256, 0, stream>>>(a, lda, rows, k, V.ea + r0, V.ba + r0, T.logT,
                                                                device_status_ptr());
   with_crt_moduli(T.n, [&](auto nm) {
-    residue_rows_kernel<decltype(nm)::value><<<dim3(rows, ceil_div(L.ldp / 8, 128)), 128, 0, stream>>>(
+    residue_rows_kernel<decltype(nm)::value><<<dim3(rows, ceil_div(k, 8 * 128)), 128, 0, stream>>>(
         a, lda, rows, k, V.ea + r0, V.ba + r0, T, V.pa + (int64_t)r0 * L.ldp, L.ldp, (int64_t)m * L.ldp);
   });
   PHPC_CUDA_TRY(cudaGetLastError());
@@ -281,7 +282,7 @@ int ozaki2_prepare_b_cols(int m, int k, int n, int c0, int cols, const double* d
   const int* pe = merge ? nullptr : V.pe + c0;
   with_crt_moduli(T.n, [&](auto nm) {
     residue_cols_kernel<decltype(nm)::value>
-        <<<dim3(ceil_div(cols, kColBlockJ), ceil_div(L.ldp, kColBlockK)), 256, 0, stream>>>(
+        <<<dim3(ceil_div(cols, kColBlockJ), ceil_div(k, kColBlockK)), 256, 0, stream>>>(
             b, ldb, k, cols, L.ldpart, pe, V.ps + c0, eb, bb, T, V.pb + (int64_t)c0 * L.ldp, L.ldp,
             (int64_t)n * L.ldp);
   });

@@ -117,6 +117,17 @@ int default_grouped_stages(const phpc_gemm_problem* problems, int count);
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
+// Row stride (in BF16 elements) of an operand plane K long. TMA needs 16-byte
+// rows; rows that start off a 32-byte sector cost the GEMM a fifth sector per
+// 128-byte box row and 1.6x its time (m = n = 3000: 695 us at K = 3000 or
+// 3016, 466 at 3040, 442 at 3008; whole 128-byte lines are another 5 %), so
+// rows are padded to 128 bytes, short ones (where that could double a plane)
+// to 32. A workspace that holds only the 16-byte layout still gets that one.
+inline int64_t plane_ld(int k, bool padded) {
+  const int64_t to = !padded ? 8 : k >= 256 ? 64 : 16;
+  return (k + to - 1) / to * to;
+}
+
 inline int ceil_div(int64_t a, int64_t b) { return static_cast<int>((a + b - 1) / b); }
 
 }  // namespace phpc

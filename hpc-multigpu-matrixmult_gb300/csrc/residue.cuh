@@ -475,7 +475,7 @@ __device__ __forceinline__ void residue_col_block(const double* __restrict__ B, 
   __syncthreads();
   const int jj = threadIdx.x >> 3, p = threadIdx.x & 7;
   const int64_t col = j0 + jj, kp = k0 + 8 * p;
-  if (col >= N || kp >= ldp) return;
+  if (col >= N || kp >= K) return;
   double v[8];
 #pragma unroll
   for (int u = 0; u < 8; ++u) v[u] = tile[8 * p + u][jj ^ (4 * (p & 3))];
