@@ -10,8 +10,8 @@
 //    ring of 2-6 stages (4 unless PHPC_DMMA_STAGES or the tuning table's
 //    "plain" entry says otherwise) with TMA (the on-device form of the reference's
 //    per-panel row/column broadcasts, src/phpc_summa.c:63-89);
-//  - consumer warps computing 32 x 32 outputs each with FP64 accumulation in
-//    registers over the whole K range, on the scalar FP64 pipe (DFMA, the
+//  - consumer warps computing 8 x 8 to 16 x 16 outputs each with FP64
+//    accumulation in registers over the whole K range, on the scalar FP64 pipe (DFMA, the
 //    default: 1.245 TFLOP/s at N = 16384, the GPU's FP64 rate) or on the FP64
 //    tensor cores (mma.sync.m16n8k4.f64, PHPC_FP64_PIPE=dmma: 1.089 TFLOP/s);
 //    both give the same bits, those of the reference's kernel;
@@ -21,6 +21,7 @@
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
+#include <type_traits>
 
 #include "phpc_dev.cuh"
 #include "phpc_host.hpp"
@@ -41,44 +42,59 @@ struct SummaGrid {
 // logical SUMMA grid in row-major order, tiles row-major inside a block.
 // Block (bi, bj) owns tile rows [bi*tm/gh, (bi+1)*tm/gh) and tile columns
 // [bj*tn/gw, (bj+1)*tn/gw).
+// Computed, not searched: block (bi, .) is the last whose first tile row is at
+// or before tile row t / tn (gh <= tm, gw <= tn).
 __device__ __forceinline__ void tile_coords(const SummaGrid& g, int t, int& rm, int& rn) {
-  for (int bi = 0; bi < g.gh; ++bi) {
-    const int r0 = (int)((int64_t)bi * g.tm / g.gh), r1 = (int)((int64_t)(bi + 1) * g.tm / g.gh);
-    for (int bj = 0; bj < g.gw; ++bj) {
-      const int c0 = (int)((int64_t)bj * g.tn / g.gw), c1 = (int)((int64_t)(bj + 1) * g.tn / g.gw);
-      const int cnt = (r1 - r0) * (c1 - c0);
-      if (t < cnt) {
-        const int w = c1 - c0;
-        rm = r0 + t / w;
-        rn = c0 + t % w;
-        return;
-      }
-      t -= cnt;
-    }
-  }
-  rm = rn = 0;
+  const int bi = static_cast<int>(((int64_t)(t / g.tn + 1) * g.gh - 1) / g.tm);
+  const int r0 = (int)((int64_t)bi * g.tm / g.gh), r1 = (int)((int64_t)(bi + 1) * g.tm / g.gh);
+  t -= r0 * g.tn;
+  const int bj = static_cast<int>(((int64_t)(t / (r1 - r0) + 1) * g.gw - 1) / g.tn);
+  const int c0 = (int)((int64_t)bj * g.tn / g.gw), c1 = (int)((int64_t)(bj + 1) * g.tn / g.gw);
+  t -= (r1 - r0) * c0;
+  rm = r0 + t / (c1 - c0);
+  rn = c0 + t % (c1 - c0);
 }
 
-template <int BM, int BN>
+// Square tiles of BT x BT outputs (16 or 32), warps of WM x WN. Each of the
+// SM's four quarters has its own FP64 pipe (half an FMA a clock), so both
+// tiles give every quarter a warp (FP64 tensor-core warps are at least
+// 16 x 8). Larger tiles buy nothing, since the pipe, not shared memory or L2,
+// is the limit: 64 x 64 tiles took 14.4 ms at N = 2048 against 14.05 for
+// 16 x 16, 128 x 128 tiles 895 ms at N = 8192 against 883 for 32 x 32, and a
+// call that leaves SMs idle at 64 x 64 is up to 8x slower (250 x 514 x 302:
+// 566 us against 73.6).
+template <int BT, bool DFMA>
 struct DmmaCfg {
-  static constexpr int kWarpsM = BM / 32, kWarpsN = BN / 32;
-  static constexpr int kConsumers = kWarpsM * kWarpsN;
+  static constexpr int BM = BT, BN = BT;
+  static constexpr int WM = BT == 32 ? 16 : DFMA ? 8 : 16;
+  static constexpr int WN = BT == 32 ? 16 : 8;
+  static constexpr int kWarpsN = BN / WN;
+  static constexpr int kConsumers = (BM / WM) * kWarpsN;
   static constexpr int kThreads = (kConsumers + 1) * 32;
   static constexpr int kStageA = BM * kBK * 8;
   static constexpr int kStageB = kBK * BN * 8;
-  static constexpr int kStageBytes = kStageA + kStageB;
+  static constexpr int kStageBytes = kStageA + kStageB;  // a multiple of 1024: A's swizzle atoms stay aligned
   static constexpr size_t smem(int stages) { return (size_t)stages * kStageBytes + 1024 /*align*/ + 256 /*barriers*/; }
 };
+
+// A's rows of 16 doubles are stored with the 128-byte swizzle: element (row,
+// k) is at 16-byte chunk (k / 2) ^ (row % 8) of its row, so that the eight
+// rows a warp reads at one k lie in different banks. Chunk c of row `row`:
+__device__ __forceinline__ const double* a_chunk(const double* sA, int row, int c) {
+  return sA + row * kBK + 2 * (c ^ (row & 7));
+}
 
 // DFMA = false: mma.sync.m16n8k4.f64 (FP64 tensor cores); true: the same
 // outputs per thread computed with scalar FP64 FMAs. Both sum every output
 // over k in increasing order with one rounding per FMA, so they give the same
 // bits (and the same bits as the reference's SIMT kernel).
-template <int BM, int BN, bool DFMA>
-__global__ void __launch_bounds__(DmmaCfg<BM, BN>::kThreads)
+template <int BT, bool DFMA>
+__global__ void __launch_bounds__(DmmaCfg<BT, DFMA>::kThreads)
     dmma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, double* C,
                      int64_t ldc, int M, int N, int K, int kpanel, SummaGrid grid, int stages, int* status) {
-  using Cfg = DmmaCfg<BM, BN>;
+  using Cfg = DmmaCfg<BT, DFMA>;
+  constexpr int BM = Cfg::BM, BN = Cfg::BN, WM = Cfg::WM, WN = Cfg::WN;
+  constexpr int NR = WM / 8, NJ = WN / 8;  // a thread's outputs: rows g + 8 r, columns 8 j + 2 tig, + 1
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int S = stages;  // ring depth, 2 .. kMaxStages (checked by the launcher)
@@ -147,13 +163,11 @@ __global__ void __launch_bounds__(DmmaCfg<BM, BN>::kThreads)
     for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
       int rm, rn;
       tile_coords(grid, t, rm, rn);
-      double acc[2][4][4];
+      double acc[NR][NJ][2];
 #pragma unroll
-      for (int i = 0; i < 2; ++i)
+      for (int r = 0; r < NR; ++r)
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-#pragma unroll
-          for (int r = 0; r < 4; ++r) acc[i][j][r] = 0.0;
+        for (int j = 0; j < NJ; ++j) acc[r][j][0] = acc[r][j][1] = 0.0;
 
       for (int ks = 0; ks < ksteps; ++ks) {
         // all lanes must agree before the warp-collective mma.sync below
@@ -162,77 +176,72 @@ __global__ void __launch_bounds__(DmmaCfg<BM, BN>::kThreads)
         const double* sA = reinterpret_cast<const double*>(smem + stage * Cfg::kStageBytes);  // [BM][16]
         const double* sB = reinterpret_cast<const double*>(smem + stage * Cfg::kStageBytes + Cfg::kStageA);  // [16][BN]
         if (DFMA) {
-#pragma unroll 1
-          for (int kk = 0; kk < kBK; ++kk) {
-            double a[2][2], b[4][2];
+#pragma unroll 2
+          for (int c = 0; c < kBK / 2; ++c) {
+            double2 a[NR];
 #pragma unroll
-            for (int i = 0; i < 2; ++i)
+            for (int r = 0; r < NR; ++r)
+              a[r] = *reinterpret_cast<const double2*>(a_chunk(sA, wm * WM + 8 * r + g, c));
 #pragma unroll
-              for (int h = 0; h < 2; ++h) a[i][h] = sA[(wm * 32 + i * 16 + g + 8 * h) * kBK + kk];
+            for (int h = 0; h < 2; ++h) {
+              double2 b[NJ];
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
+              for (int j = 0; j < NJ; ++j)
+                b[j] = *reinterpret_cast<const double2*>(&sB[(2 * c + h) * BN + wn * WN + j * 8 + 2 * tig]);
 #pragma unroll
-              for (int c = 0; c < 2; ++c) b[j][c] = sB[kk * BN + wn * 32 + j * 8 + 2 * tig + c];
+              for (int r = 0; r < NR; ++r)
 #pragma unroll
-            for (int i = 0; i < 2; ++i)
-#pragma unroll
-              for (int j = 0; j < 4; ++j)
-#pragma unroll
-                for (int h = 0; h < 2; ++h)
-#pragma unroll
-                  for (int c = 0; c < 2; ++c) acc[i][j][2 * h + c] = fma(a[i][h], b[j][c], acc[i][j][2 * h + c]);
+                for (int j = 0; j < NJ; ++j) {
+                  acc[r][j][0] = fma(h ? a[r].y : a[r].x, b[j].x, acc[r][j][0]);
+                  acc[r][j][1] = fma(h ? a[r].y : a[r].x, b[j].y, acc[r][j][1]);
+                }
+            }
           }
         } else {
 #pragma unroll
-        for (int kk = 0; kk < kBK; kk += 4) {
-          double a[2][2], b[4];
+          for (int kk = 0; kk < kBK; kk += 4) {
+            double a[NR], b[NJ];
 #pragma unroll
-          for (int i = 0; i < 2; ++i) {
-            const int row = wm * 32 + i * 16 + g;
-            a[i][0] = sA[row * kBK + kk + tig];
-            a[i][1] = sA[(row + 8) * kBK + kk + tig];
+            for (int r = 0; r < NR; ++r) a[r] = a_chunk(sA, wm * WM + 8 * r + g, (kk + tig) >> 1)[tig & 1];
+#pragma unroll
+            for (int j = 0; j < NJ; ++j) b[j] = sB[(kk + tig) * BN + wn * WN + j * 8 + g];
+#pragma unroll
+            for (int r = 0; r + 1 < NR; r += 2)
+#pragma unroll
+              for (int j = 0; j < NJ; ++j)
+                asm volatile(
+                    "mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
+                    : "+d"(acc[r][j][0]), "+d"(acc[r][j][1]), "+d"(acc[r + 1][j][0]), "+d"(acc[r + 1][j][1])
+                    : "d"(a[r]), "d"(a[r + 1]), "d"(b[j]));
           }
-#pragma unroll
-          for (int j = 0; j < 4; ++j) b[j] = sB[(kk + tig) * BN + wn * 32 + j * 8 + g];
-#pragma unroll
-          for (int i = 0; i < 2; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-              asm volatile(
-                  "mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
-                  : "+d"(acc[i][j][0]), "+d"(acc[i][j][1]), "+d"(acc[i][j][2]), "+d"(acc[i][j][3])
-                  : "d"(a[i][0]), "d"(a[i][1]), "d"(b[j]));
-        }
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty[stage]);
         if (++stage == S) { stage = 0; phase ^= 1; }
       }
       if (!ok) break;
-      // Epilogue: C += tile (rows g and g+8 of each m16 block, two adjacent columns).
+      // Epilogue: C += tile.
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
+      for (int r = 0; r < NR; ++r) {
+        const int64_t row = (int64_t)rm * BM + wm * WM + 8 * r + g;
+        if (row >= M) continue;
+        double* crow = C + row * ldc;
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int64_t row = (int64_t)rm * BM + wm * 32 + i * 16 + g + h * 8;
-          if (row >= M) continue;
-          double* crow = C + row * ldc;
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const int col = rn * BN + wn * 32 + j * 8 + 2 * tig;
-            if (col < N) crow[col] += acc[i][j][2 * h];
-            if (col + 1 < N) crow[col + 1] += acc[i][j][2 * h + 1];
-          }
+        for (int j = 0; j < NJ; ++j) {
+          const int col = rn * BN + wn * WN + j * 8 + 2 * tig;
+          if (col < N) crow[col] += acc[r][j][0];
+          if (col + 1 < N) crow[col + 1] += acc[r][j][1];
         }
       }
     }
   }
 }
 
-template <int BM, int BN, bool DFMA>
+template <int BT, bool DFMA>
 int launch_dmma(int m, int k, int n, const double* dA, int64_t lda, const double* dB, int64_t ldb, double* dC,
                 int64_t ldc, int gw, int gh, int kpanel, cudaStream_t stream) {
-  using Cfg = DmmaCfg<BM, BN>;
+  using Cfg = DmmaCfg<BT, DFMA>;
+  constexpr int BM = Cfg::BM, BN = Cfg::BN;
   const DeviceInfo* dev = current_device();
   if (!dev) return PHPC_ERR_CUDA;
   CUtensorMap tmA, tmB;
@@ -242,7 +251,7 @@ int launch_dmma(int m, int k, int n, const double* dA, int64_t lda, const double
   const uint64_t dimsB[2] = {(uint64_t)n, (uint64_t)k};
   const uint64_t strB[1] = {(uint64_t)ldb * 8};
   const uint32_t boxB[2] = {BN, kBK};
-  if (!encode_tiled(&tmA, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, dA, dimsA, strA, boxA, CU_TENSOR_MAP_SWIZZLE_NONE) ||
+  if (!encode_tiled(&tmA, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, dA, dimsA, strA, boxA, CU_TENSOR_MAP_SWIZZLE_128B) ||
       !encode_tiled(&tmB, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, dB, dimsB, strB, boxB, CU_TENSOR_MAP_SWIZZLE_NONE))
     return PHPC_ERR_CUDA;
   SummaGrid g;
@@ -251,7 +260,7 @@ int launch_dmma(int m, int k, int n, const double* dA, int64_t lda, const double
   g.gh = std::min(gh, g.tm);
   g.gw = std::min(gw, g.tn);
   const int ntiles = g.tm * g.tn;
-  auto kern = dmma_gemm_kernel<BM, BN, DFMA>;
+  auto kern = dmma_gemm_kernel<BT, DFMA>;
   const int stages = default_plain_stages(m, k, n);
   if (stages < 2 || stages > kMaxStages) return PHPC_ERR_ARG;
   const size_t smem = Cfg::smem(stages);
@@ -275,22 +284,30 @@ bool fp64_pipe_is_dfma() {
   return !(pipe && strcmp(pipe, "dmma") == 0);
 }
 
-// Tile shape: 128 x 128 when there are at least two waves of such tiles,
-// else 64 x 64 so that small problems still spread over the SMs.
+// Tile side: a call takes as long as the SM with the most outputs (padding
+// included), ceil(tiles / SMs) x BT^2, so the smaller tile is never behind by
+// load (N = 1024 in 64 x 64 tiles: 2104 us, 2 tiles on some SMs, 1 on others;
+// in 16 x 16: 1813). From 128 tiles of 32 x 32 an SM that difference is under
+// 1 % and the larger tile's fewer loads count for more (N = 4096, 108 tiles an
+// SM: 16 111.0 ms, 32 111.6; N = 8192: 887 and 883). PHPC_DMMA_TILE = 16 forces
+// the one, any other number the other.
+int plain_tile(int m, int n, int sms) {
+  if (const char* force = getenv("PHPC_DMMA_TILE")) return atoi(force) == 16 ? 16 : 32;
+  return (int64_t)ceil_div(m, 32) * ceil_div(n, 32) >= (int64_t)128 * sms ? 32 : 16;
+}
+
 int dgemm_dmma(int m, int k, int n, const double* dA, int64_t lda, const double* dB, int64_t ldb, double* dC,
                int64_t ldc, int gw, int gh, int kpanel, cudaStream_t stream) {
   const DeviceInfo* dev = current_device();
   if (!dev) return PHPC_ERR_CUDA;
   if (dev->cc_major != 10 || dev->cc_minor != 3) return PHPC_ERR_UNSUPPORTED;
-  const int64_t tiles128 = (int64_t)ceil_div(m, 128) * ceil_div(n, 128);
-  const char* force = getenv("PHPC_DMMA_TILE");
-  const bool big = force ? atoi(force) == 128 : tiles128 >= 2 * dev->sm_count;
-  const bool dfma = fp64_pipe_is_dfma();
-  if (big)
-    return dfma ? launch_dmma<128, 128, true>(m, k, n, dA, lda, dB, ldb, dC, ldc, gw, gh, kpanel, stream)
-                : launch_dmma<128, 128, false>(m, k, n, dA, lda, dB, ldb, dC, ldc, gw, gh, kpanel, stream);
-  return dfma ? launch_dmma<64, 64, true>(m, k, n, dA, lda, dB, ldb, dC, ldc, gw, gh, kpanel, stream)
-              : launch_dmma<64, 64, false>(m, k, n, dA, lda, dB, ldb, dC, ldc, gw, gh, kpanel, stream);
+  auto launch = [&](auto tile) {
+    constexpr int T = decltype(tile)::value;
+    return fp64_pipe_is_dfma() ? launch_dmma<T, true>(m, k, n, dA, lda, dB, ldb, dC, ldc, gw, gh, kpanel, stream)
+                               : launch_dmma<T, false>(m, k, n, dA, lda, dB, ldb, dC, ldc, gw, gh, kpanel, stream);
+  };
+  return plain_tile(m, n, dev->sm_count) == 16 ? launch(std::integral_constant<int, 16>())
+                                                : launch(std::integral_constant<int, 32>());
 }
 
 }  // namespace phpc
