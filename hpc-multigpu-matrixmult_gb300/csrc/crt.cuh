@@ -19,19 +19,19 @@ __host__ __device__ constexpr int crt_digits(int n) {
   return kDigits[n];
 }
 
-// What the residue GEMMs store per element and modulus (a 16-bit value): not
-// the residue r_i of the product but t_i = r_i ((M / m_i)^-1 mod m_i) mod m_i,
-// symmetric (|t_i| <= 182), plus kCrtTBias. (A's residue planes carry the
+// What the residue GEMMs store per element and modulus: not the residue r_i
+// of the product but t_i = r_i ((M / m_i)^-1 mod m_i) mod m_i, symmetric
+// (|t_i| <= 182), as a BF16 value (exact). (A's residue planes carry the
 // factor (M / m_i)^-1 mod m_i, so the GEMM's sums are t_i mod m_i.) Then
 // sum_i t_i (M / m_i) = y (mod M), so the reconstruction needs no
 // per-modulus multiplication.
-constexpr int kCrtTBias = 256;
 
-// Constants of the reconstruction on FP32 limbs (crt_limbs_quad), each value
+// Constants of the reconstruction on FP32 limbs (crt_limbs_quad), the floats
 // in both lanes of a packed f32x2 operation.
 struct CrtLimbs {
   int np;                                 // digits of the largest M / m_i (5 .. 10)
-  float2 unbias;                          // -(2^23 + kCrtTBias)
+  int pow[3];                             // 1, 2^13, 2^26: factors the compiler must not turn into shifts
+                                          // (the multiply-adds run beside the shift and logic pipe)
   float2 cw[3];                           // 2^(13 j) / M rounded to float, j = np - 1, np - 2, np - 3
   float2 P[kCrtMaxModuli][kCrtMaxLimbs];  // balanced 13-bit digits of M / m_i, least significant first
   float2 negM[kCrtMaxLimbs + 1];          // balanced 13-bit digits of M, negated
@@ -205,12 +205,12 @@ __device__ __forceinline__ double crt_round(uint32_t (&l)[5], const CrtTable& T,
 template <int NMOD>
 __device__ __forceinline__ double crt_value(const uint32_t (&rr)[kCrtMaxModuli], const CrtTable& T, int fast,
                                             int& shift) {
-  // rr[i] is the stored t_i + kCrtTBias; acc = sum_i (t_i mod m_i) (M / m_i),
+  // rr[i] is the stored t_i (BF16 bits); acc = sum_i (t_i mod m_i) (M / m_i),
   // 32-bit limbs accumulated in 64 bits (no overflow: 15 x 2^9 x 2^32 < 2^45)
   uint64_t a0 = 0, a1 = 0, a2 = 0, a3 = 0;
 #pragma unroll
   for (int i = 0; i < NMOD; ++i) {
-    const int32_t t = static_cast<int32_t>(rr[i]) - kCrtTBias;
+    const int32_t t = __float2int_rn(__uint_as_float(rr[i] << 16));
     const uint32_t r = static_cast<uint32_t>(t < 0 ? t + static_cast<int32_t>(T.m[i]) : t);
     a0 += static_cast<uint64_t>(r) * T.W[i][0];
     a1 += static_cast<uint64_t>(r) * T.W[i][1];
@@ -270,58 +270,63 @@ __device__ __forceinline__ double crt_add_i128(double c, uint64_t lo, uint64_t h
   return c + ldexp(sign ? -m : m, e - 52 + x);
 }
 
+// A reconstructed integer y = w[0] + w[1] 2^52 + w[2] 2^104, the words signed
+// and overlapping (|w[0]|, |w[1]| < 2^63).
+struct CrtWords {
+  int64_t w[3];
+};
+
+__device__ __forceinline__ int64_t mad_wide(int a, int b, int64_t c) {
+  int64_t d;
+  asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(d) : "r"(a), "r"(b), "l"(c));
+  return d;
+}
+
 // The one-step CRT of four adjacent elements on FP32 limbs: two pairs, each
 // pair in the two lanes of packed f32x2 operations, both pairs computed in
 // one pass over the moduli so that each modulus's constants are read once
-// for the four elements. w[p][i] holds the stored t_i + kCrtTBias of pair p
-// for modulus i (its first element in the low 16 bits, the second in the
-// high 16 bits). Valid when every result satisfies |y| / M <= 1/2 - 1/32
-// (CrtTable::fast); gives the y of crt_value as 128-bit two's complement
-// integers (lo[e], hi[e]), e = 2 p + lane. Every step except the quotient
-// estimate is exact in FP32 (all values are integers below 2^24):
-//  1. t_i read as the float 2^23 + kCrtTBias + t_i (the stored bits under the
-//     exponent of 2^23), less 2^23 + kCrtTBias: one exact add;
-//     sum_i t_i (M / m_i) = y (mod M);
+// for the four elements. w[p][i] holds the stored t_i of pair p for modulus i
+// (BF16, its first element in the low 16 bits, the second in the high 16
+// bits). Valid when every result satisfies |y| / M <= 1/2 - 1/32
+// (CrtTable::fast); gives the y of crt_value, element e = 2 p + lane. Every
+// step except the quotient estimate is exact in FP32 (all values are integers
+// below 2^24):
+//  1. t_i from its bits; sum_i t_i (M / m_i) = y (mod M);
 //  2. S_j = sum_i t_i P_ij over the balanced 13-bit digits P_ij of M / m_i
-//     (|P_ij| <= 2^12, |S_j| <= 15 182 2^12 < 2^24);
+//     (|P_ij| <= 2^12, |S_j| <= 15 182 2^12 < 2^23.5);
 //  3. q = round(sum_i t_i / m_i) from the top three limb sums,
 //     est = sum_j S_j fl(2^(13 j) / M) (|est| <= 7.5, error below 2^-19; the
 //     lower limbs weigh below 2^-27); exact under the fast path's margin;
-//  4. Y_j = S_j - q M_j (|Y_j| < 2^24), the limbs of y = sum_j Y_j 2^(13 j);
-//  5. carries: h_j = round(Y_j 2^-13), digits d_j = (Y_j - h_j 2^13) + h_(j-1)
-//     (|d_j| < 2^13), read out as integers through the rounding constant
-//     1.5 2^23; four digits make a 52-bit chunk (int64), and
-//     y = A + B 2^52 + C 2^104 for the chunks A, B, C.
+//  4. Y_j = S_j - q M_j (|Y_j| < 2^23.5), the limbs of y = sum_j Y_j 2^(13 j),
+//     converted to integers;
+//  5. four limbs make a word (|word| < 2^23.5 (2^39 + 2^26 + ..) < 2^63),
+//     by 32 x 32 + 64-bit multiply-adds.
+// (The limbs were once carried into small digits in FP32 and assembled and
+// rounded in 128-bit integers, 213 of the kernel's 349 issue cycles a warp
+// element on the integer pipe, its limit; see crt_round_add for the rounding.)
 // NMOD = T.n, the number of moduli; NP = T.L.np = crt_digits(NMOD), the
 // number of digits of the largest M / m_i.
 template <int NMOD>
 __device__ __forceinline__ void crt_limbs_quad(const uint32_t (&w)[2][kCrtMaxModuli], const CrtTable& T,
-                                               uint64_t (&lo)[4], uint64_t (&hi)[4]) {
+                                               CrtWords (&out)[4]) {
   constexpr int NP = crt_digits(NMOD);
   const float2 kRound = make_float2(12582912.0f, 12582912.0f), kUnround = make_float2(-12582912.0f, -12582912.0f);
-  const float2 kDigit = make_float2(0x1p-13f, 0x1p-13f), kNegBase = make_float2(-8192.0f, -8192.0f);
   float2 S[2][NP];
 #pragma unroll
   for (int p = 0; p < 2; ++p)
 #pragma unroll
     for (int j = 0; j < NP; ++j) S[p][j] = make_float2(0.0f, 0.0f);
-  const float2 unbias = T.L.unbias;
 #pragma unroll
   for (int i = 0; i < NMOD; ++i) {
-    {
-      float2 t[2];
+    float2 t[2];
 #pragma unroll
-      for (int p = 0; p < 2; ++p) {
-        const float2 tb = make_float2(__uint_as_float(0x4B000000u | (w[p][i] & 0xFFFFu)),
-                                      __uint_as_float(0x4B000000u | (w[p][i] >> 16)));
-        t[p] = __fadd2_rn(tb, unbias);
-      }
+    for (int p = 0; p < 2; ++p)
+      t[p] = make_float2(__uint_as_float(w[p][i] << 16), __uint_as_float(w[p][i] & 0xFFFF0000u));
 #pragma unroll
-      for (int j = 0; j < NP; ++j) {
-        const float2 pij = T.L.P[i][j];
-        S[0][j] = __ffma2_rn(t[0], pij, S[0][j]);
-        S[1][j] = __ffma2_rn(t[1], pij, S[1][j]);
-      }
+    for (int j = 0; j < NP; ++j) {
+      const float2 pij = T.L.P[i][j];
+      S[0][j] = __ffma2_rn(t[0], pij, S[0][j]);
+      S[1][j] = __ffma2_rn(t[1], pij, S[1][j]);
     }
   }
 #pragma unroll
@@ -330,41 +335,72 @@ __device__ __forceinline__ void crt_limbs_quad(const uint32_t (&w)[2][kCrtMaxMod
     est = __ffma2_rn(S[p][NP - 2], T.L.cw[1], est);
     est = __ffma2_rn(S[p][NP - 3], T.L.cw[2], est);
     const float2 q = __fadd2_rn(__fadd2_rn(est, kRound), kUnround);
-    int d0[12], d1[12];  // digits; those above NP + 1 are zero
+    int Y[2][12];  // the limbs; those above NP are zero
 #pragma unroll
-    for (int j = 0; j < 12; ++j) d0[j] = d1[j] = 0;
-    float2 hprev = make_float2(0.0f, 0.0f);
+    for (int j = 0; j < 12; ++j) {
+      if (j <= NP) {
+        const float2 y = j < NP ? __ffma2_rn(q, T.L.negM[j], S[p][j]) : __fmul2_rn(q, T.L.negM[NP]);
+        Y[0][j] = __float2int_rn(y.x);
+        Y[1][j] = __float2int_rn(y.y);
+      } else {
+        Y[0][j] = Y[1][j] = 0;
+      }
+    }
 #pragma unroll
-    for (int j = 0; j <= NP; ++j) {
-      const float2 y = j < NP ? __ffma2_rn(q, T.L.negM[j], S[p][j]) : __fmul2_rn(q, T.L.negM[NP]);
-      const float2 h = __fadd2_rn(__ffma2_rn(y, kDigit, kRound), kUnround);
-      const float2 d = __fadd2_rn(__fadd2_rn(__ffma2_rn(h, kNegBase, y), hprev), kRound);
-      d0[j] = __float_as_int(d.x) - 0x4B400000;
-      d1[j] = __float_as_int(d.y) - 0x4B400000;
-      hprev = h;
-    }
-    {
-      const float2 d = __fadd2_rn(hprev, kRound);
-      d0[NP + 1] = __float_as_int(d.x) - 0x4B400000;
-      d1[NP + 1] = __float_as_int(d.y) - 0x4B400000;
-    }
-    // 52-bit chunks of four digits: |chunk| < 2^52 (int64 exact)
-    auto chunk = [](const int (&d)[12], int j0) -> int64_t {
-      const int32_t a = d[j0] + d[j0 + 1] * 8192, b = d[j0 + 2] + d[j0 + 3] * 8192;
-      return static_cast<int64_t>(a) + static_cast<int64_t>(b) * 67108864;
-    };
+    for (int l = 0; l < 2; ++l)
 #pragma unroll
-    for (int l = 0; l < 2; ++l) {
-      const int(&d)[12] = l ? d1 : d0;
-      const int64_t A = chunk(d, 0), B = chunk(d, 4), C = chunk(d, 8);
-      // y = A + B 2^52 + C 2^104 modulo 2^128
-      const uint64_t b_lo = static_cast<uint64_t>(B) << 52;
-      const int e = 2 * p + l;
-      lo[e] = static_cast<uint64_t>(A) + b_lo;
-      hi[e] = static_cast<uint64_t>(A >> 63) + static_cast<uint64_t>(B >> 12) + (static_cast<uint64_t>(C) << 40) +
-              (lo[e] < b_lo ? 1 : 0);
-    }
+      for (int g = 0; g < 3; ++g) {
+        const int(&y)[12] = Y[l];
+        int64_t v = 0;
+        if (4 * g + 3 <= NP) v = static_cast<int64_t>(static_cast<uint64_t>(static_cast<uint32_t>(y[4 * g + 3]) << 7) << 32);
+        if (4 * g + 2 <= NP) v = mad_wide(y[4 * g + 2], T.L.pow[2], v);
+        if (4 * g + 1 <= NP) v = mad_wide(y[4 * g + 1], T.L.pow[1], v);
+        if (4 * g <= NP) v = mad_wide(y[4 * g], T.L.pow[0], v);
+        out[2 * p + l].w[g] = v;
+      }
   }
+}
+
+// c + y 2^x for a reconstructed y, |y| <= M (1/2 - 1/32): y rounded once to
+// double (to nearest even), the sum rounded once.
+//
+// Up to 13 moduli |y| < 2^108.6: with V = floor(y / 2^52) (64 bits) and A its
+// low 52 bits, y = B 2^58 + A', B = V >> 6 (|B| < 2^51), 0 <= A' < 2^58. Both
+// halves become doubles through their bits: 2^58 + A' with A''s low 6 bits
+// folded into one sticky bit, and (B - 1) 2^58 by one exact subtraction of a
+// constant; their sum is y's one rounding (for |y| >= 2^60 half an ulp lies
+// above the sticky bit). |V| < 2^32 (a zero, a strong cancellation) is rare:
+// there V is exact in double and so is A. Three FP64 additions a value: 48
+// cycles of the SM's FP64 pipe a warp, below the 58 that a warp's 42 bytes an
+// element take at DRAM speed. The kernel: N = 4096 158 -> 130 us (5.4 TB/s),
+// 16384 2.8 -> 2.24 ms, 512-problem batch 1.81 -> 1.59 ms.
+template <int NMOD>
+__device__ __forceinline__ double crt_round_add(double c, const CrtWords& y, int x) {
+  if (NMOD <= 13) {
+    const uint64_t w0 = static_cast<uint64_t>(y.w[0]);
+    const int64_t V = static_cast<int64_t>(static_cast<uint64_t>(y.w[1]) + static_cast<uint64_t>(y.w[0] >> 52) +
+                                           (static_cast<uint64_t>(y.w[2]) << 52));
+    double r;
+    if (static_cast<uint32_t>(static_cast<int32_t>(V >> 32) + 1) <= 1u) {
+      const double a = __longlong_as_double(static_cast<long long>((w0 & ((1ull << 52) - 1)) | (0x433ull << 52))) - 0x1p52;
+      r = fma(static_cast<double>(V), 0x1p52, a);
+      if (r == 0.0) return c + 0.0;
+    } else {
+      const uint32_t h0 = static_cast<uint32_t>(w0 >> 32), l0 = static_cast<uint32_t>(w0);
+      const uint32_t lo = __funnelshift_r(l0, h0, 6) | ((l0 & 63u) != 0 ? 1u : 0u);
+      const uint32_t hi = ((h0 >> 6) & 0x3FFFu) | ((static_cast<uint32_t>(V) << 14) & 0xFC000u) | ((1023u + 58u) << 20);
+      const int64_t zb = (V >> 6) + static_cast<int64_t>((1023ull + 52 + 58) << 52 | 1ull << 51);
+      const double xb = __longlong_as_double(zb) - (0x1.8p52 + 1.0) * 0x1p58;  // (B - 1) 2^58
+      r = xb + __hiloint2double(static_cast<int>(hi), static_cast<int>(lo));
+    }
+    return crt_add_scaled(c, r, x);
+  }
+  // y modulo 2^128
+  const uint64_t b_lo = static_cast<uint64_t>(y.w[1]) << 52;
+  const uint64_t lo = static_cast<uint64_t>(y.w[0]) + b_lo;
+  const uint64_t hi = static_cast<uint64_t>(y.w[0] >> 63) + static_cast<uint64_t>(y.w[1] >> 12) +
+                      (static_cast<uint64_t>(y.w[2]) << 40) + (lo < b_lo ? 1 : 0);
+  return crt_add_i128(c, lo, hi, x);
 }
 
 // *c += v * 2^(shift + e): the CRT result of one element applied to C

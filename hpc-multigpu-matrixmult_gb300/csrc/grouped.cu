@@ -268,10 +268,9 @@ inline int64_t crt_blocks_of(int64_t crt_units) { return (crt_units + kCrtBlockU
 // unit (written with the plan); a warp walks on from it (a block's units
 // span at most kCrtBlockUnits problems).
 template <int NMOD>
-__global__ void __launch_bounds__(32 * kCrtBlockUnits) g_crt_kernel(const GSplitProb* __restrict__ P,
-                                                                   const int* __restrict__ first, int count,
-                                                                   int total_units,
-                                                                   const __grid_constant__ ModTable T) {
+__global__ void __launch_bounds__(32 * kCrtBlockUnits, crt_min_blocks(NMOD, true))
+    g_crt_kernel(const GSplitProb* __restrict__ P, const int* __restrict__ first, int count, int total_units,
+                 const __grid_constant__ ModTable T) {
   const int u = blockIdx.x * kCrtBlockUnits + (threadIdx.x >> 5);
   if (u >= total_units) return;
   int pi = first[blockIdx.x];

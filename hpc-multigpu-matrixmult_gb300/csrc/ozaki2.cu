@@ -161,11 +161,10 @@ __global__ void __launch_bounds__(256) residue_cols_kernel(const double* __restr
 
 // C[i][j] += C_int * 2^(ea[i] - ba[i] + eb[j] - bb[j]), C_int recovered from the residues.
 template <int NMOD>
-__global__ void __launch_bounds__(128) crt_kernel(const uint16_t* __restrict__ R, int64_t ldr, int64_t rplane, int M,
-                                                  int N, const int* __restrict__ ea, const int* __restrict__ ba,
-                                                  const int* __restrict__ eb, const int* __restrict__ bb,
-                                                  const __grid_constant__ ModTable T, double* __restrict__ C,
-                                                  int64_t ldc) {
+__global__ void __launch_bounds__(128, crt_min_blocks(NMOD, false))
+    crt_kernel(const uint16_t* __restrict__ R, int64_t ldr, int64_t rplane, int M, int N, const int* __restrict__ ea,
+               const int* __restrict__ ba, const int* __restrict__ eb, const int* __restrict__ bb,
+               const __grid_constant__ ModTable T, double* __restrict__ C, int64_t ldc) {
   const int64_t row = blockIdx.x;
   const int64_t c0 = ((int64_t)blockIdx.y * blockDim.x + threadIdx.x) * kCrtCols;
   if (row >= M || c0 >= N) return;

@@ -126,8 +126,7 @@ inline ModTable make_table(int nmod, int k) {
   int np = 0;
   for (int i = 0; i < nmod; ++i) np = std::max(np, digits(M / kModuli[i], T.crt.L.P[i], kCrtMaxLimbs));
   T.crt.L.np = np;
-  const float ub = -(8388608.0f + static_cast<float>(kCrtTBias));
-  T.crt.L.unbias = make_float2(ub, ub);
+  for (int j = 0; j < 3; ++j) T.crt.L.pow[j] = 1 << (13 * j);
   for (int j = 0; j < 3; ++j) {
     const float c = static_cast<float>(std::ldexp(1.0, 13 * (np - 1 - j)) / static_cast<double>(M));
     T.crt.L.cw[j] = make_float2(c, c);
@@ -490,6 +489,13 @@ __device__ __forceinline__ void residue_col_block(const double* __restrict__ B, 
 // 128-byte run of each plane row and a warp's loads cover 4 columns of 8 rows.
 constexpr int kColBlockK = 64, kColBlockJ = 32;
 
+// Blocks of 128 threads per SM the CRT kernels are held to up to 13 moduli
+// (above, the compiler's choice, 5): they wait on their loads of the residue
+// planes, so warps in flight count for more than a few spilled registers. The
+// grouped kernel holds its problem's fields too (7 blocks: batch 6.88 ms, 8:
+// 7.07, no bound, 5 blocks: 7.17).
+constexpr int crt_min_blocks(int nmod, bool grouped) { return nmod > 13 ? 5 : grouped ? 7 : 8; }
+
 constexpr int kCrtCols = 4;  // consecutive columns per thread (one 8-byte load per residue plane)
 
 // Calls f(std::integral_constant<int, n>()) for the number of moduli n
@@ -532,19 +538,19 @@ __device__ __forceinline__ void crt_cols(const uint16_t* __restrict__ rp, int64_
       w[0][i] = rw[i].x;
       w[1][i] = rw[i].y;
     }
-    uint64_t lo[kCrtCols], hi[kCrtCols];
-    crt_limbs_quad<NMOD>(w, T, lo, hi);
+    CrtWords y[kCrtCols];
+    crt_limbs_quad<NMOD>(w, T, y);
     if (ncols == kCrtCols) {
       double cv[kCrtCols];
 #pragma unroll
       for (int c = 0; c < kCrtCols; ++c) cv[c] = cp[c];
 #pragma unroll
       for (int c = 0; c < kCrtCols; ++c)
-        cp[c] = crt_add_i128(cv[c], lo[c], hi[c], row_shift + max(ebp[c], -20000) - bbp[c]);
+        cp[c] = crt_round_add<NMOD>(cv[c], y[c], row_shift + max(ebp[c], -20000) - bbp[c]);
     } else {
 #pragma unroll
       for (int c = 0; c < kCrtCols; ++c)
-        if (c < ncols) cp[c] = crt_add_i128(cp[c], lo[c], hi[c], row_shift + max(ebp[c], -20000) - bbp[c]);
+        if (c < ncols) cp[c] = crt_round_add<NMOD>(cp[c], y[c], row_shift + max(ebp[c], -20000) - bbp[c]);
     }
     return;
   }

@@ -86,13 +86,10 @@ __device__ __forceinline__ float2 reduce_pair_f32(float2 x, float m, float invm)
 // What the residue GEMM stores for two integer-valued floats |x| < 2^24, the
 // products' sums (A's residues carry the factor (M / m)^-1 mod m, so x = t
 // mod m for the t the CRT combines): t = x mod m, symmetric (|t| <= 0.51 m,
-// at most 182), plus kCrtTBias (crt.cuh), as two 16-bit values (lo in the low
-// half) read from the mantissas of 2^23 + kCrtTBias + t.
-__device__ __forceinline__ uint32_t crt_t_pair_u16(float x0, float x1, float m, float invm) {
+// at most 182), as two BF16 values (exact; lo in the low half).
+__device__ __forceinline__ uint32_t crt_t_pair(float x0, float x1, float m, float invm) {
   const float2 t = reduce_pair_f32(make_float2(x0, x1), m, invm);
-  const float bias = 8388608.0f + static_cast<float>(kCrtTBias);
-  const float2 b = __fadd2_rn(t, make_float2(bias, bias));
-  return __byte_perm(__float_as_uint(b.x), __float_as_uint(b.y), 0x5410);
+  return __byte_perm(__float_as_uint(t.x), __float_as_uint(t.y), 0x7632);
 }
 
 struct TcArgs {
@@ -672,7 +669,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                 uint32_t w[4];
 #pragma unroll
                 for (int e = 0; e < 4; ++e)
-                  w[e] = crt_t_pair_u16(__int_as_float(acc[h + 8 * c + 2 * e]), __int_as_float(acc[h + 8 * c + 2 * e + 1]),
+                  w[e] = crt_t_pair(__int_as_float(acc[h + 8 * c + 2 * e]), __int_as_float(acc[h + 8 * c + 2 * e + 1]),
                                         mf, invm);
                 tq[lane * 8 + (c ^ (lane & 7))] = make_uint4(w[0], w[1], w[2], w[3]);
               }
