@@ -24,6 +24,7 @@
 // multiply-add per element per diagonal): this GPU's FP64 rate is ~1 TFLOP/s,
 // ~2000x below its BF16 tensor rate.
 #include <algorithm>
+#include <atomic>
 #include <cstdlib>
 #include <mutex>
 
@@ -92,6 +93,75 @@ PairList ozaki_pairs(int s) {
 
 }  // namespace
 
+namespace {
+
+template <int BN>
+cudaLaunchConfig_t ksplit_config(int split, cudaLaunchAttribute* attr) {
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = static_cast<unsigned>(split);
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(static_cast<unsigned>(split), 1, 1);
+  cfg.blockDim = dim3(kTcThreads, 1, 1);
+  cfg.dynamicSmemBytes = TcCfg<BN>::kSmem;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cfg;
+}
+
+constexpr int kMaxKsplit = 8;
+
+// Clusters of `split` K-splitting CTAs that run at one time (the clusters of
+// one GPC share its SMs, so this is below SMs / split); asked once a device.
+template <int BN>
+int ksplit_clusters(int split, const DeviceInfo* dev) {
+  constexpr int kDevices = 64;
+  static std::atomic<int> cached[kDevices][kMaxKsplit + 1];
+  if (dev->ordinal < 0 || dev->ordinal >= kDevices) return 0;
+  std::atomic<int>& c = cached[dev->ordinal][split];
+  int n = c.load(std::memory_order_relaxed);
+  if (n == 0) {
+    auto kern = tc_slice_gemm_kernel<BN, kF32, false, 1, true>;
+    cudaLaunchAttribute attr[1];
+    const cudaLaunchConfig_t cfg = ksplit_config<BN>(split, attr);
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcCfg<BN>::kSmem) !=
+            cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      n = 0;
+    }
+    c.store(n + 1, std::memory_order_relaxed);
+  } else {
+    --n;
+  }
+  return n;
+}
+
+// CTAs (one cluster) that share a tile of the 3xBF16 GEMM along K when its
+// 128 x 256 tiles (whatever the tile width in use, so that the sums do not
+// depend on it) leave SMs idle: the most, up to 8, with which every tile still
+// runs at once; a second wave costs more than the split gives. Whole calls,
+// unsplit / chosen / one more: 1000 x 777 x 1530 (48 tiles) 49.4 us, 37.1
+// with 2, 50 with 3 (144 CTAs in clusters of 3 do not fit at once); N = 1024
+// (32 tiles) 53.5, 32.2 with 4, 47.5 with 5; 700 x 3000 x 900 117, 48.3 with 5,
+// 66 with 8; 128 x 4096 x 512 140, 41 with 8. Below 48 steps (K <= 448) there
+// is little to share and the shares' additions would cost accuracy; from there
+// the error is 0.43 to 0.7 of the unsplit one (1000 x 777 x 1530: 2.1e-7
+// against 3.7e-7), since a share flushes its accumulator twice as often.
+// PHPC_F32_KSPLIT = 1..8 forces it.
+template <int BN>
+int f32_ksplit(int m, int n, int steps, const DeviceInfo* dev) {
+  const char* env = getenv("PHPC_F32_KSPLIT");
+  if (env && atoi(env) >= 1 && atoi(env) <= kMaxKsplit) return std::min(atoi(env), steps);
+  const int64_t tiles = (int64_t)ceil_div(m, kTcBM) * ceil_div(n, 256);
+  for (int s = kMaxKsplit; s > 1; --s)
+    if (tiles * s <= dev->sm_count && steps >= 48 && steps / s >= 4 && tiles <= ksplit_clusters<BN>(s, dev)) return s;
+  return 1;
+}
+
+}  // namespace
+
 // Launches the tcgen05 slice GEMM over bf16 planes (shared with the 3xBF16
 // and modular paths).
 template <int BN, int MODE>
@@ -150,6 +220,20 @@ int launch_tc_slice_gemm(const void* planesA, const void* planesB, int nplanesA,
   }
   const int64_t units =
       (cluster == 1 ? (int64_t)a.tm * a.tn : (int64_t)((a.tm + 1) / 2) * a.tn) * (a.split_pairs ? pairs.n : 1);
+  if constexpr (MODE == kF32) {
+    a.ksplit = f32_ksplit<BN>(m, n, pairs.n * ceil_div(k, kTcBK), dev);
+    if (a.ksplit > 1) {
+      auto kern = tc_slice_gemm_kernel<BN, MODE, false, 1, true>;
+      if (!tc_regs_ok(reinterpret_cast<const void*>(kern))) return PHPC_ERR_UNSUPPORTED;
+      PHPC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::kSmem));
+      cudaLaunchAttribute attr[1];
+      cudaLaunchConfig_t cfg = ksplit_config<BN>(a.ksplit, attr);
+      cfg.gridDim = dim3(static_cast<unsigned>(a.tm * a.tn * a.ksplit), 1, 1);
+      cfg.stream = stream;
+      PHPC_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, tmA, tmB, pairs, a, TcGroupTable{}));
+      return PHPC_OK;
+    }
+  }
   if (cluster == 1) {
     auto kern = tc_slice_gemm_kernel<BN, MODE>;
     if (!tc_regs_ok(reinterpret_cast<const void*>(kern))) return PHPC_ERR_UNSUPPORTED;

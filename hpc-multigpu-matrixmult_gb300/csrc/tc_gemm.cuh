@@ -55,6 +55,7 @@ constexpr int kTcMaxPairs = 64;
 constexpr int kTcChunkSteps = 16;      // kOzaki: 16 x 64 = 1024 products (|d| <= 128) per exact f32 chunk
 constexpr int kTcResidueChunkSteps = 8;  // kResidue: 8 x 64 = 512 products (|r| <= 181) per exact f32 chunk
 constexpr int kTcF32ChunkSteps = 8;    // kF32: flush to round-to-nearest registers every 512 products
+constexpr int kTcKsplitChunkSteps = 4;  // ... every 256 where K is split: pays for the shares' extra additions
 constexpr int kTcFoldChunks = 127;     // kOzaki: 127 chunks of |v| <= 2^24 keep |int32 sum| < 2^31
 constexpr int kTcEpiWarps = 8;
 constexpr int kTcFirstEpiWarp = 4;
@@ -106,6 +107,7 @@ struct TcArgs {
   int64_t rplane;             // kResidue: plane stride in elements
   int split_pairs;            // kResidue: a work unit is one (tile, modulus), moduli outer
   int stages;                 // K-stages of the ring in use, 2 .. TcCfg::kStages (other values: kStages)
+  int ksplit;                 // KSPLIT: CTAs (one cluster) per tile
   int k_serpentine;           // kResidue: every other round of units walks K from the end (see the producer)
 };
 
@@ -258,12 +260,21 @@ __device__ __forceinline__ double fold_add(double c, int32_t s, int x) {
   return c + ldexp(static_cast<double>(s), x);  // subnormal or overflowing terms
 }
 
-template <int BN, int MODE, bool GROUPED = false, int CLUSTER = 1>
+// Byte offset of 16-byte chunk c of row r of a KSPLIT CTA's sums (rows of BN
+// floats) in shared memory; chunks are swizzled so that the rows a
+// quarter-warp writes lie in different banks.
+template <int BN>
+__device__ __forceinline__ uint32_t ksplit_chunk(int r, int c) {
+  return static_cast<uint32_t>(r * BN * 4 + 16 * (c ^ (r & 7)));
+}
+
+template <int BN, int MODE, bool GROUPED = false, int CLUSTER = 1, bool KSPLIT = false>
 __global__ void __launch_bounds__(kTcThreads, 1)
     tc_slice_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                          const __grid_constant__ PairList pairs, const __grid_constant__ TcArgs args,
                          const __grid_constant__ TcGroupTable gt) {
   static_assert(CLUSTER == 1 || (CLUSTER == 2 && !GROUPED), "the CTA pair computes tiles of one problem");
+  static_assert(!KSPLIT || (MODE == kF32 && CLUSTER == 1 && !GROUPED), "K is split in the FP32 GEMM only");
   using Cfg = TcCfg<BN, CLUSTER>;
   // The shared-memory layout is that of the deepest ring; the ring in use has
   // S stages (the tuning table's pipeline depth).
@@ -288,8 +299,12 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   // Work units: 128 x BN tiles (CLUSTER = 1) or 256 x BN pair tiles (CLUSTER = 2).
   const uint32_t crank = CLUSTER > 1 ? cluster_ctarank() : 0u;
   const bool leader = crank == 0;
-  const int unit0 = CLUSTER > 1 ? static_cast<int>(cluster_id_x()) : static_cast<int>(blockIdx.x);
-  const int ustride = CLUSTER > 1 ? static_cast<int>(nclusters_x()) : static_cast<int>(gridDim.x);
+  const int unit0 = CLUSTER > 1 || KSPLIT ? static_cast<int>(cluster_id_x()) : static_cast<int>(blockIdx.x);
+  const int ustride = CLUSTER > 1 || KSPLIT ? static_cast<int>(nclusters_x()) : static_cast<int>(gridDim.x);
+  // KSPLIT (one tile per cluster): this CTA's share [ks0, ks1) of the tile's steps
+  const int krank = KSPLIT ? static_cast<int>(cluster_ctarank()) : 0;
+  const int ksteps = KSPLIT ? pairs.n * ((args.K + kTcBK - 1) / kTcBK) : 0;
+  const int ks0 = KSPLIT ? ksteps * krank / args.ksplit : 0, ks1 = KSPLIT ? ksteps * (krank + 1) / args.ksplit : 0;
   const int ntiles = GROUPED ? gt.ntiles : (CLUSTER > 1 ? (args.tm + 1) / 2 : args.tm) * args.tn;
   int* status = args.status;
 
@@ -395,7 +410,9 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         const bool rev = serp && (round & 1);
         for (int pi = p0; pi < p1 && ok; ++pi) {
           const int pa = pairs.a[pi], pb = pairs.b[pi];
-          for (int kb = 0; kb < job.nk; ++kb) {
+          const int kb0 = KSPLIT ? min(max(ks0 - pi * job.nk, 0), job.nk) : 0;
+          const int kb1 = KSPLIT ? min(max(ks1 - pi * job.nk, 0), job.nk) : job.nk;
+          for (int kb = kb0; kb < kb1; ++kb) {
             if (!wait_parity(&empty[stage], phase ^ 1, status, 11)) { ok = false; break; }
             uint8_t* sa = smem + stage * Cfg::kStageBytes;
             const int kx = (rev ? job.nk - 1 - kb : kb) * kTcBK;
@@ -468,8 +485,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             while (gend < p1 && pairs.g[gend] == pairs.g[gstart]) ++gend;
           else
             gend = p1;
-          const int total = (gend - gstart) * nk;
-          const int chunk = MODE == kOzaki ? kTcChunkSteps : MODE == kResidue ? kTcResidueChunkSteps : kTcF32ChunkSteps;
+          const int total = KSPLIT ? ks1 - ks0 : (gend - gstart) * nk;
+          const int chunk = MODE == kOzaki ? kTcChunkSteps : MODE == kResidue ? kTcResidueChunkSteps : KSPLIT ? kTcKsplitChunkSteps : kTcF32ChunkSteps;
           for (int done = 0; done < total && ok; done += chunk) {
             const int len = min(chunk, total - done);
             if (!wait_parity(&tempty[buf], tphase[buf] ^ 1, status, 12)) { ok = false; break; }
@@ -515,6 +532,11 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       const uint64_t t0 = globaltimer_ns();
       while (!mbar_try_wait(daddr, 0) && globaltimer_ns() - t0 < PHPC_WAIT_LIMIT_NS) {}
     }
+  }
+  if (KSPLIT) {  // the epilogue warps' two cluster barriers
+    __syncwarp();
+    cluster_sync();
+    cluster_sync();
   }
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kTcRegsHigh));
@@ -566,8 +588,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
           while (gend < p1 && pairs.g[gend] == pairs.g[gstart]) ++gend;
         else
           gend = p1;
-        const int total = (gend - gstart) * job.nk;
-        const int chunk = MODE == kOzaki ? kTcChunkSteps : MODE == kResidue ? kTcResidueChunkSteps : kTcF32ChunkSteps;
+        const int total = KSPLIT ? ks1 - ks0 : (gend - gstart) * job.nk;
+        const int chunk = MODE == kOzaki ? kTcChunkSteps : MODE == kResidue ? kTcResidueChunkSteps : KSPLIT ? kTcKsplitChunkSteps : kTcF32ChunkSteps;
         const int nchunks = (total + chunk - 1) / chunk;
         for (int c = 0; c < nchunks && ok; ++c) {
           // all lanes must agree before the warp-collective tcgen05.ld below
@@ -699,6 +721,15 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             for (int u = 0; u < HALF; ++u) acc[u] = 0;
             continue;
           }
+          if (KSPLIT) {
+            // every MMA of this CTA has read its operands: the ring is free
+            const int r = quad * 32 + lane;
+#pragma unroll
+            for (int c = 0; c < HALF / 4; ++c)
+              *reinterpret_cast<int4*>(smem + ksplit_chunk<BN>(r, half * (HALF / 4) + c)) =
+                  make_int4(acc[4 * c], acc[4 * c + 1], acc[4 * c + 2], acc[4 * c + 3]);
+            continue;
+          }
           // Write the warp's 32 rows x HALF columns out, 32 columns at a time,
           // transposed through shared memory so that a warp touches one
           // contiguous 32-element run of a row per access.
@@ -756,6 +787,60 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         }
         gstart = gend;
       }
+    }
+    if (KSPLIT) {
+      cluster_sync();  // every CTA's sums are in its shared memory
+      TcJob job;
+      tc_job<GROUPED, CLUSTER>(unit0, args, &tmA, &tmB, gt, crank, job);
+      const uint32_t base = smem_u32(smem);
+      // this CTA's rows, four 16-byte chunks a thread at a time, four CTAs' sums
+      // of each in flight, their C values on the way meanwhile
+      const int r0 = kTcBM * krank / args.ksplit, r1 = kTcBM * (krank + 1) / args.ksplit;
+      constexpr int kChunks = BN / 4, kBatch = 4;
+      float* Cf = static_cast<float*>(job.C);
+      for (int i0 = ew * 32 + lane; i0 < (r1 - r0) * kChunks; i0 += kBatch * kTcEpiWarps * 32) {
+        float cv[kBatch][4];
+        float4 sum[kBatch];
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u) {
+          const int i = i0 + u * kTcEpiWarps * 32, r = r0 + i / kChunks, col = job.rn * BN + 4 * (i % kChunks);
+          const int64_t row = (int64_t)job.rm * kTcBM + r;
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            cv[u][e] = r < r1 && row < job.M && col + e < job.N ? Cf[row * job.ldc + col + e] : 0.f;
+        }
+        for (int q0 = 0; q0 < args.ksplit; q0 += 4) {
+          float4 v[4][kBatch];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const uint32_t peer = mapa_shared(base, min(q0 + q, args.ksplit - 1));
+#pragma unroll
+            for (int u = 0; u < kBatch; ++u) {
+              const int i = min(i0 + u * kTcEpiWarps * 32, (r1 - r0) * kChunks - 1);
+              if (q0 + q < args.ksplit)
+                v[q][u] = ld_shared_cluster_f4(peer + ksplit_chunk<BN>(r0 + i / kChunks, i % kChunks));
+            }
+          }
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            if (q0 + q < args.ksplit)
+#pragma unroll
+              for (int u = 0; u < kBatch; ++u)
+                sum[u] = q0 + q == 0 ? v[q][u]
+                                     : make_float4(sum[u].x + v[q][u].x, sum[u].y + v[q][u].y, sum[u].z + v[q][u].z,
+                                                   sum[u].w + v[q][u].w);
+        }
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u) {
+          const int i = i0 + u * kTcEpiWarps * 32, r = r0 + i / kChunks, col = job.rn * BN + 4 * (i % kChunks);
+          const int64_t row = (int64_t)job.rm * kTcBM + r;
+          const float s4[4] = {sum[u].x, sum[u].y, sum[u].z, sum[u].w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            if (r < r1 && row < job.M && col + e < job.N) Cf[row * job.ldc + col + e] = cv[u][e] + s4[e];
+        }
+      }
+      cluster_sync();  // no CTA leaves while a peer reads its sums
     }
   }
 
