@@ -39,63 +39,76 @@ namespace phpc {
 
 namespace {
 
-// One warp per row of A: ea[i] = max_k e(A[i][k]) and the row's grid width.
-__global__ void scan_rows_grid_kernel(const double* __restrict__ A, int64_t lda, int M, int K, int* __restrict__ ea,
-                                      int* __restrict__ ba, float logT, int* status) {
-  const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (row >= M) return;
-  const double* a = A + row * lda;
-  NormAcc acc;
-  bool nf = false;
-  norm_row_lane(a, K, threadIdx.x & 31, acc, nf);
-  acc = norm_warp(acc);
-  if ((threadIdx.x & 31) == 0) {
-    ea[row] = acc.e;
-    ba[row] = grid_bits(acc.s, K, logT);
-  }
-  if (__any_sync(0xffffffffu, nf) && (threadIdx.x & 31) == 0) record_error(status, PHPC_ERR_NONFINITE);
-}
+// The A side (rows) and the B side (columns) of one operand preparation.
+// Either may be empty (rows / cols = 0): the two kernels below run one side
+// or both in one launch, A's blocks first.
+struct PrepRows {
+  const double* A;
+  int64_t lda;
+  int rows;
+  int* ea;
+  int* ba;
+  uint16_t* planes;  // [n][.][ldp]
+  int64_t plane_stride;
+};
+struct PrepCols {
+  const double* B;
+  int64_t ldb;
+  int cols;
+  int64_t ldpart;
+  int* pe;
+  float* ps;
+  int* eb;
+  int* bb;
+  uint16_t* planes;  // [n][.][ldp], transposed
+  int64_t plane_stride;
+  int merge;  // the split merges the scan's chunks itself
+};
 
-// Column scan, part 1: block (strip of 32 columns, chunk of 256 rows); warp w
-// sums rows 32 w .. + 31 of the chunk, and warp 0 merges the eight slices in
-// order into pe / ps [chunk][n]. A column's chain is 32 FMAs with 16 loads in
-// flight, and even N = 256 has 8 blocks; one thread per column and 256 rows
-// took 53-59 us at every size up to N = 4096 (the chain's latency) and 410 us
-// at N = 16384, against 4 us at N = 256, 5.5 at 1024, 22 at 4096 and 292 at
-// 16384 (7.3 TB/s) for this.
-__global__ void __launch_bounds__(256) scan_cols_part_kernel(const double* __restrict__ B, int64_t ldb, int K, int N,
-                                                             int64_t ldpart, int* __restrict__ pe,
-                                                             float* __restrict__ ps, int* status) {
+constexpr int kPrepThreads = 256;
+constexpr int kScanRowsPerBlock = kPrepThreads / 32;  // one warp per row
+
+// Row blocks: one warp per row of A: ea[i] = max_k e(A[i][k]) and the row's
+// grid width. Column blocks (scan part 1): strip of 32 columns, chunk of 256
+// rows; warp w sums rows 32 w .. + 31 of the chunk, and warp 0 merges the eight
+// slices in order into pe / ps [chunk][n]. A column's chain is 32 FMAs with 16
+// loads in flight, and even N = 256 has 8 blocks; one thread per column and
+// 256 rows took 53-59 us at every size up to N = 4096 (the chain's latency)
+// and 410 us at N = 16384, against 4 us at N = 256, 5.5 at 1024, 22 at 4096
+// and 292 at 16384 (7.3 TB/s) for this.
+__global__ void __launch_bounds__(kPrepThreads) scan_kernel(const PrepRows a, const PrepCols b, int row_blocks,
+                                                            int strips, int K, float logT, int* status) {
   __shared__ int se[8][32];
   __shared__ float ss[8][32];
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  const int64_t col = (int64_t)blockIdx.x * 32 + l;
-  const int k0 = blockIdx.y * kNormChunk + w * kNormSlice;
   NormAcc acc;
   bool nf = false;
-  if (col < N && k0 < K) norm_col_slice(B, ldb, col, k0, K, acc, nf);
+  if (static_cast<int>(blockIdx.x) < row_blocks) {
+    const int64_t row = (int64_t)blockIdx.x * kScanRowsPerBlock + w;
+    if (row >= a.rows) return;
+    norm_row_lane(a.A + row * a.lda, K, l, acc, nf);
+    acc = norm_warp(acc);
+    if (l == 0) {
+      a.ea[row] = acc.e;
+      a.ba[row] = grid_bits(acc.s, K, logT);
+    }
+    if (__any_sync(0xffffffffu, nf) && l == 0) record_error(status, PHPC_ERR_NONFINITE);
+    return;
+  }
+  const int blk = blockIdx.x - row_blocks, chunk = blk / strips;
+  const int64_t col = (int64_t)(blk - chunk * strips) * 32 + l;
+  const int k0 = chunk * kNormChunk + w * kNormSlice;
+  if (col < b.cols && k0 < K) norm_col_slice(b.B, b.ldb, col, k0, K, acc, nf);
   se[w][l] = acc.e;
   ss[w][l] = acc.s;
   if (nf) record_error(status, PHPC_ERR_NONFINITE);
   __syncthreads();
-  if (w != 0 || col >= N) return;
+  if (w != 0 || col >= b.cols) return;
   acc = NormAcc{};
 #pragma unroll
   for (int u = 0; u < 8; ++u) norm_merge(acc, NormAcc{se[u][l], ss[u][l]});
-  pe[blockIdx.y * ldpart + col] = acc.e;
-  ps[blockIdx.y * ldpart + col] = acc.s;
-}
-
-// A residue planes [n][M][ldp]: blockIdx.x = row, each thread 8 consecutive k.
-template <int NMOD>
-__global__ void residue_rows_kernel(const double* __restrict__ A, int64_t lda, int M, int K,
-                                    const int* __restrict__ ea, const int* __restrict__ ba,
-                                    const __grid_constant__ ModTable T, uint16_t* __restrict__ planes, int64_t ldp,
-                                    int64_t plane_stride) {
-  const int64_t row = blockIdx.x;
-  const int64_t k0 = ((int64_t)blockIdx.y * blockDim.x + threadIdx.x) * 8;
-  if (row >= M || k0 >= K) return;
-  residue_row_piece<NMOD>(A + row * lda, K, ea[row], ba[row], T, planes + row * ldp, plane_stride, k0);
+  b.pe[chunk * b.ldpart + col] = acc.e;
+  b.ps[chunk * b.ldpart + col] = acc.s;
 }
 
 // Column scan, part 2: a block merges the chunks of 32 columns, warp p those
@@ -122,41 +135,63 @@ __global__ void __launch_bounds__(256) scan_cols_merge_kernel(int K, int N, int6
   bb[col] = grid_bits(acc.s, K, logT);
 }
 
-// Up to this many chunks (K <= 1024) the column split merges them itself: a
-// merge kernel is 3-4 us of a small call, the merge in every block of the
+// Up to this many chunks (K <= 1024) the split merges them itself: a merge
+// kernel is 3-4 us of a small call, the merge in every block of the
 // split 0.6 us of 11 at N = 1024 (but 22 us of 120 at N = 4096, 0.9 ms of
 // 2.4 at 16384).
 constexpr int kMergeInSplit = 4;
 
-// B residue planes, transposed ([n][N][ldp]): one kColBlockK x kColBlockJ
-// block per 256-thread CTA (residue.cuh). With pe the eight threads of a
-// column merge its chunks into the exponent and grid width, and the first row
-// of blocks stores them in eb / bb for the CRT; without, eb / bb are there.
+// Row blocks: A residue planes [n][M][ldp], a thread per row piece (8
+// consecutive k of one row). A block takes 256 consecutive pieces of a row,
+// rows first (the rows' pieces of one range of k together: 1.43 ms at N =
+// 16384 against 1.44-1.65 with a row's ranges together); what is left of the
+// rows, or rows shorter than that, is numbered row by row, so that the blocks
+// are full. Column blocks: B residue planes, transposed
+// ([n][N][ldp]), one kColBlockK x kColBlockJ block each (residue.cuh); with
+// b.merge the eight threads of a column merge its chunks into the exponent
+// and grid width, and the first row of blocks stores them in eb / bb for the
+// CRT; without, eb / bb are there.
 template <int NMOD>
-__global__ void __launch_bounds__(256) residue_cols_kernel(const double* __restrict__ B, int64_t ldb, int K, int N,
-                                                           int64_t ldpart, const int* __restrict__ pe,
-                                                           const float* __restrict__ ps, int* eb, int* bb,
-                                                           const __grid_constant__ ModTable T,
-                                                           uint16_t* __restrict__ planes, int64_t ldp,
-                                                           int64_t plane_stride) {
+__global__ void __launch_bounds__(kPrepThreads, 4)
+    residue_split_kernel(const PrepRows a, const PrepCols b, int row_blocks, int strips, int K, int64_t ldp,
+                         const __grid_constant__ ModTable T) {
   __shared__ double tile[kColBlockK][kColBlockJ];
-  const int64_t j0 = (int64_t)blockIdx.x * kColBlockJ, col = j0 + (threadIdx.x >> 3);
+  if (static_cast<int>(blockIdx.x) < row_blocks) {
+    const int per_row = (K + 7) >> 3, ranges = per_row / kPrepThreads, left = per_row - ranges * kPrepThreads;
+    const int64_t blk = blockIdx.x, full = (int64_t)a.rows * ranges;
+    int64_t row, piece;
+    if (blk < full) {
+      const int range = static_cast<int>(blk / a.rows);
+      row = blk - (int64_t)range * a.rows;
+      piece = range * kPrepThreads + threadIdx.x;
+    } else {
+      const int64_t t = (blk - full) * kPrepThreads + threadIdx.x, pieces = (int64_t)a.rows * left;
+      if (t >= pieces) return;
+      row = pieces <= UINT32_MAX ? static_cast<uint32_t>(t) / static_cast<uint32_t>(left) : t / left;
+      piece = ranges * kPrepThreads + (t - row * left);
+    }
+    residue_row_piece<NMOD>(a.A + row * a.lda, K, a.ea[row], a.ba[row], T, a.planes + row * ldp, a.plane_stride,
+                            piece * 8);
+    return;
+  }
+  const int blk = blockIdx.x - row_blocks, kb = blk / strips;
+  const int64_t j0 = (int64_t)(blk - kb * strips) * kColBlockJ, col = j0 + (threadIdx.x >> 3);
   int e, bits;
-  if (pe) {
+  if (b.merge) {
     const int chunks = (K + kNormChunk - 1) / kNormChunk;
-    const NormAcc acc = norm_merge_chunks8(pe, ps, ldpart, col, col < N ? chunks : 0, threadIdx.x & 7);
+    const NormAcc acc = norm_merge_chunks8(b.pe, b.ps, b.ldpart, col, col < b.cols ? chunks : 0, threadIdx.x & 7);
     e = acc.e;
     bits = grid_bits(acc.s, K, T.logT);
-    if (blockIdx.y == 0 && col < N && (threadIdx.x & 7) == 0) {
-      eb[col] = e;
-      bb[col] = bits;
+    if (kb == 0 && col < b.cols && (threadIdx.x & 7) == 0) {
+      b.eb[col] = e;
+      b.bb[col] = bits;
     }
   } else {
-    e = col < N ? eb[col] : 0;
-    bits = col < N ? bb[col] : 0;
+    e = col < b.cols ? b.eb[col] : 0;
+    bits = col < b.cols ? b.bb[col] : 0;
   }
-  residue_col_block<NMOD>(B, ldb, K, N, j0, (int64_t)blockIdx.y * kColBlockK, e, bits, T, planes, ldp, plane_stride,
-                          tile);
+  residue_col_block<NMOD>(b.B, b.ldb, K, b.cols, j0, (int64_t)kb * kColBlockK, e, bits, T, b.planes, ldp,
+                          b.plane_stride, tile);
 }
 
 // C[i][j] += C_int * 2^(ea[i] - ba[i] + eb[j] - bb[j]), C_int recovered from the residues.
@@ -238,6 +273,45 @@ size_t ozaki2_workspace_bytes(int m, int k, int n, int nmod) { return ozaki2_lay
 
 int ozaki2_bits(int nmod, int k) { return make_table(nmod, k).bits; }
 
+namespace {
+
+// Scans and residue splits of a's rows and b's columns (either side may be
+// empty): two launches, three when the chunks of the column scan are merged
+// between them.
+int prepare_operands(const PrepRows& a, PrepCols b, int k, int64_t ldp, const ModTable& T, cudaStream_t stream) {
+  const int strips = ceil_div(b.cols, 32), chunks = ceil_div(k, kNormChunk);
+  const int scan_rows = ceil_div(a.rows, kScanRowsPerBlock);
+  const int ranges = ceil_div(k, 8) / kPrepThreads, left = ceil_div(k, 8) - ranges * kPrepThreads;
+  const int split_rows = a.rows * ranges + ceil_div((int64_t)a.rows * left, kPrepThreads);
+  b.merge = chunks <= kMergeInSplit;
+  scan_kernel<<<scan_rows + strips * chunks, kPrepThreads, 0, stream>>>(a, b, scan_rows, strips, k, T.logT,
+                                                                        device_status_ptr());
+  if (b.cols > 0 && !b.merge)
+    scan_cols_merge_kernel<<<strips, 256, 0, stream>>>(k, b.cols, b.ldpart, b.pe, b.ps, b.eb, b.bb, T.logT);
+  with_crt_moduli(T.n, [&](auto nm) {
+    residue_split_kernel<decltype(nm)::value>
+        <<<split_rows + strips * ceil_div(k, kColBlockK), kPrepThreads, 0, stream>>>(a, b, split_rows, strips, k, ldp,
+                                                                                     T);
+  });
+  PHPC_CUDA_TRY(cudaGetLastError());
+  return PHPC_OK;
+}
+static_assert(kColBlockJ == 32, "scan strips are the split's column blocks");
+
+PrepRows prep_rows(int m, int r0, int rows, const double* dA, int64_t lda, const Ozaki2Layout& L,
+                   const Ozaki2Views& V) {
+  return PrepRows{dA + (int64_t)r0 * lda, lda,         rows, V.ea + r0, V.ba + r0, V.pa + (int64_t)r0 * L.ldp,
+                  (int64_t)m * L.ldp};
+}
+
+PrepCols prep_cols(int n, int c0, int cols, const double* dB, int64_t ldb, const Ozaki2Layout& L,
+                   const Ozaki2Views& V) {
+  return PrepCols{dB + c0,   ldb,       cols,      L.ldpart, V.pe + c0, V.ps + c0,
+                  V.eb + c0, V.bb + c0, V.pb + (int64_t)c0 * L.ldp, (int64_t)n * L.ldp, 0};
+}
+
+}  // namespace
+
 // Rows [r0, r0 + rows) of A (an m x k operand, dA its row 0): exponent and
 // grid scan, and residue split into the planes of the full problem.
 int ozaki2_prepare_a_rows(int m, int r0, int rows, int k, int n, const double* dA, int64_t lda, int nmod, void* ws,
@@ -247,16 +321,7 @@ int ozaki2_prepare_a_rows(int m, int r0, int rows, int k, int n, const double* d
   const int rc = ozaki2_views(m, k, n, nmod, ws, ws_bytes, L, V);
   if (rc != PHPC_OK) return rc;
   if (r0 < 0 || rows <= 0 || r0 + rows > m) return PHPC_ERR_ARG;
-  const ModTable T = make_table(nmod, k);
-  const double* a = dA + (int64_t)r0 * lda;
-  scan_rows_grid_kernel<<<ceil_div(rows, 8), 256, 0, stream>>>(a, lda, rows, k, V.ea + r0, V.ba + r0, T.logT,
-                                                               device_status_ptr());
-  with_crt_moduli(T.n, [&](auto nm) {
-    residue_rows_kernel<decltype(nm)::value><<<dim3(rows, ceil_div(k, 8 * 128)), 128, 0, stream>>>(
-        a, lda, rows, k, V.ea + r0, V.ba + r0, T, V.pa + (int64_t)r0 * L.ldp, L.ldp, (int64_t)m * L.ldp);
-  });
-  PHPC_CUDA_TRY(cudaGetLastError());
-  return PHPC_OK;
+  return prepare_operands(prep_rows(m, r0, rows, dA, lda, L, V), PrepCols{}, k, L.ldp, make_table(nmod, k), stream);
 }
 
 // Columns [c0, c0 + cols) of B (k x n, dB its column 0): exponent and grid
@@ -268,25 +333,7 @@ int ozaki2_prepare_b_cols(int m, int k, int n, int c0, int cols, const double* d
   const int rc = ozaki2_views(m, k, n, nmod, ws, ws_bytes, L, V);
   if (rc != PHPC_OK) return rc;
   if (c0 < 0 || cols <= 0 || c0 + cols > n) return PHPC_ERR_ARG;
-  const ModTable T = make_table(nmod, k);
-  const double* b = dB + c0;
-  scan_cols_part_kernel<<<dim3(ceil_div(cols, 32), ceil_div(k, kNormChunk)), 256, 0, stream>>>(
-      b, ldb, k, cols, L.ldpart, V.pe + c0, V.ps + c0, device_status_ptr());
-  int* eb = V.eb + c0;
-  int* bb = V.bb + c0;
-  const bool merge = ceil_div(k, kNormChunk) > kMergeInSplit;
-  if (merge)
-    scan_cols_merge_kernel<<<ceil_div(cols, 32), 256, 0, stream>>>(k, cols, L.ldpart, V.pe + c0, V.ps + c0, eb, bb,
-                                                                  T.logT);
-  const int* pe = merge ? nullptr : V.pe + c0;
-  with_crt_moduli(T.n, [&](auto nm) {
-    residue_cols_kernel<decltype(nm)::value>
-        <<<dim3(ceil_div(cols, kColBlockJ), ceil_div(k, kColBlockK)), 256, 0, stream>>>(
-            b, ldb, k, cols, L.ldpart, pe, V.ps + c0, eb, bb, T, V.pb + (int64_t)c0 * L.ldp, L.ldp,
-            (int64_t)n * L.ldp);
-  });
-  PHPC_CUDA_TRY(cudaGetLastError());
-  return PHPC_OK;
+  return prepare_operands(PrepRows{}, prep_cols(n, c0, cols, dB, ldb, L, V), k, L.ldp, make_table(nmod, k), stream);
 }
 
 // B (k x n): exponent and grid scan, and residue split.
@@ -303,11 +350,23 @@ int ozaki2_prepare2(int m, int k, int n, const double* dA, int64_t lda, const do
   return rc;
 }
 
-// The same on one caller stream: B's scans and split run on this thread's
-// side stream beside A's (both are memory-bound; run together, one's ramp-up
-// and tail overlap the other's), and the caller's stream waits for them.
+// The same on one caller stream. Small operands (below 32 MB together, and K
+// <= 1024: no merge kernel between scan and split) share the two launches:
+// the fork and join cost more than the overlap gives (N = 256 53 -> 42 us,
+// 1537 x 1000 x 2311 169.7 -> 168.5, but 4096 x 512 x 4096 360 -> 364). Above,
+// B's scans and split run on this thread's side stream beside A's (both are
+// memory-bound; run together, one's ramp-up and tail overlap the other's), and
+// the caller's stream waits for them.
 int ozaki2_prepare_on(int m, int k, int n, const double* dA, int64_t lda, const double* dB, int64_t ldb, int nmod,
                       void* ws, size_t ws_bytes, cudaStream_t stream) {
+  if (ceil_div(k, kNormChunk) <= kMergeInSplit && ((int64_t)m + n) * k < (4 << 20)) {
+    Ozaki2Layout L;
+    Ozaki2Views V;
+    const int rc = ozaki2_views(m, k, n, nmod, ws, ws_bytes, L, V);
+    if (rc != PHPC_OK) return rc;
+    return prepare_operands(prep_rows(m, 0, m, dA, lda, L, V), prep_cols(n, 0, n, dB, ldb, L, V), k, L.ldp,
+                            make_table(nmod, k), stream);
+  }
   const cudaStream_t side = side_stream();
   if (!side || !stream_fork(stream, side)) return ozaki2_prepare2(m, k, n, dA, lda, dB, ldb, nmod, ws, ws_bytes, stream, stream);
   int rc = ozaki2_prepare2(m, k, n, dA, lda, dB, ldb, nmod, ws, ws_bytes, stream, side);
