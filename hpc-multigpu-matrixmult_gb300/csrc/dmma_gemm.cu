@@ -264,10 +264,14 @@ int launch_dmma(int m, int k, int n, const double* dA, int64_t lda, const double
   const int stages = default_plain_stages(m, k, n);
   if (stages < 2 || stages > kMaxStages) return PHPC_ERR_ARG;
   const size_t smem = Cfg::smem(stages);
-  PHPC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  int per_sm = 1;
-  PHPC_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, Cfg::kThreads, smem));
-  per_sm = std::max(1, per_sm);
+  static PerDevice blocks_per_sm[kMaxStages + 1];
+  int per_sm = blocks_per_sm[stages].get(dev->ordinal);
+  if (per_sm == 0) {
+    PHPC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::smem(kMaxStages)));
+    PHPC_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, Cfg::kThreads, smem));
+    per_sm = std::max(1, per_sm);
+    blocks_per_sm[stages].set(dev->ordinal, per_sm);
+  }
   const int nblocks = std::min(ntiles, dev->sm_count * per_sm);
   kern<<<nblocks, Cfg::kThreads, smem, stream>>>(tmA, tmB, dC, ldc, m, n, k, kpanel, g, stages,
                                                                              device_status_ptr());

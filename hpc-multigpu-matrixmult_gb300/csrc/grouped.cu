@@ -450,12 +450,8 @@ int launch_grouped_gemm(const phpc_grouped_plan* pl, cudaStream_t stream) {
 }
 
 template <int BN, int MODE>
-int prepare_grouped_gemm() {
-  using Cfg = TcCfg<BN>;
-  auto kern = tc_slice_gemm_kernel<BN, MODE, true>;
-  if (!tc_regs_ok(reinterpret_cast<const void*>(kern))) return PHPC_ERR_UNSUPPORTED;
-  PHPC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::kSmem));
-  return PHPC_OK;
+int prepare_grouped_gemm(const DeviceInfo* dev) {
+  return tc_ready<tc_slice_gemm_kernel<BN, MODE, true>>(dev, TcCfg<BN>::kSmem);
 }
 
 int run_grouped(const phpc_grouped_plan* pl, cudaStream_t stream) {
@@ -692,9 +688,9 @@ int grouped_plan_create(phpc_grouped_plan** out, const phpc_gemm_problem* proble
     }
   if (rc == PHPC_OK) {
     if (modular)
-      rc = pl->bn == 128 ? prepare_grouped_gemm<128, kResidue>() : prepare_grouped_gemm<256, kResidue>();
+      rc = pl->bn == 128 ? prepare_grouped_gemm<128, kResidue>(dev) : prepare_grouped_gemm<256, kResidue>(dev);
     else
-      rc = pl->bn == 128 ? prepare_grouped_gemm<128, kOzaki>() : prepare_grouped_gemm<256, kOzaki>();
+      rc = pl->bn == 128 ? prepare_grouped_gemm<128, kOzaki>(dev) : prepare_grouped_gemm<256, kOzaki>(dev);
   }
   if (rc == PHPC_OK && !device_status_ptr()) rc = PHPC_ERR_CUDA;  // resolved now, not during a graph capture
   if (rc == PHPC_OK &&

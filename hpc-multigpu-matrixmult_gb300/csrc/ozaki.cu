@@ -24,7 +24,6 @@
 // multiply-add per element per diagonal): this GPU's FP64 rate is ~1 TFLOP/s,
 // ~2000x below its BF16 tensor rate.
 #include <algorithm>
-#include <atomic>
 #include <cstdlib>
 #include <mutex>
 
@@ -116,25 +115,18 @@ constexpr int kMaxKsplit = 8;
 // one GPC share its SMs, so this is below SMs / split); asked once a device.
 template <int BN>
 int ksplit_clusters(int split, const DeviceInfo* dev) {
-  constexpr int kDevices = 64;
-  static std::atomic<int> cached[kDevices][kMaxKsplit + 1];
-  if (dev->ordinal < 0 || dev->ordinal >= kDevices) return 0;
-  std::atomic<int>& c = cached[dev->ordinal][split];
-  int n = c.load(std::memory_order_relaxed);
-  if (n == 0) {
-    auto kern = tc_slice_gemm_kernel<BN, kF32, false, 1, true>;
-    cudaLaunchAttribute attr[1];
-    const cudaLaunchConfig_t cfg = ksplit_config<BN>(split, attr);
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcCfg<BN>::kSmem) !=
-            cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
-      cudaGetLastError();
-      n = 0;
-    }
-    c.store(n + 1, std::memory_order_relaxed);
-  } else {
-    --n;
+  static PerDevice cached[kMaxKsplit + 1];  // clusters + 1
+  int n = cached[split].get(dev->ordinal);
+  if (n > 0) return n - 1;
+  constexpr auto kern = tc_slice_gemm_kernel<BN, kF32, false, 1, true>;
+  cudaLaunchAttribute attr[1];
+  const cudaLaunchConfig_t cfg = ksplit_config<BN>(split, attr);
+  if (tc_ready<kern>(dev, TcCfg<BN>::kSmem) != PHPC_OK ||
+      cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    n = 0;
   }
+  cached[split].set(dev->ordinal, n + 1);
   return n;
 }
 
@@ -223,9 +215,8 @@ int launch_tc_slice_gemm(const void* planesA, const void* planesB, int nplanesA,
   if constexpr (MODE == kF32) {
     a.ksplit = f32_ksplit<BN>(m, n, pairs.n * ceil_div(k, kTcBK), dev);
     if (a.ksplit > 1) {
-      auto kern = tc_slice_gemm_kernel<BN, MODE, false, 1, true>;
-      if (!tc_regs_ok(reinterpret_cast<const void*>(kern))) return PHPC_ERR_UNSUPPORTED;
-      PHPC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::kSmem));
+      constexpr auto kern = tc_slice_gemm_kernel<BN, MODE, false, 1, true>;
+      if (const int rc = tc_ready<kern>(dev, Cfg::kSmem); rc != PHPC_OK) return rc;
       cudaLaunchAttribute attr[1];
       cudaLaunchConfig_t cfg = ksplit_config<BN>(a.ksplit, attr);
       cfg.gridDim = dim3(static_cast<unsigned>(a.tm * a.tn * a.ksplit), 1, 1);
@@ -235,9 +226,8 @@ int launch_tc_slice_gemm(const void* planesA, const void* planesB, int nplanesA,
     }
   }
   if (cluster == 1) {
-    auto kern = tc_slice_gemm_kernel<BN, MODE>;
-    if (!tc_regs_ok(reinterpret_cast<const void*>(kern))) return PHPC_ERR_UNSUPPORTED;
-    PHPC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::kSmem));
+    constexpr auto kern = tc_slice_gemm_kernel<BN, MODE>;
+    if (const int rc = tc_ready<kern>(dev, Cfg::kSmem); rc != PHPC_OK) return rc;
     const int grid = static_cast<int>(std::min<int64_t>(units, dev->sm_count));
     kern<<<grid, kTcThreads, Cfg::kSmem, stream>>>(tmA, tmB, pairs, a, TcGroupTable{});
     PHPC_CUDA_TRY(cudaGetLastError());
@@ -245,9 +235,8 @@ int launch_tc_slice_gemm(const void* planesA, const void* planesB, int nplanesA,
   }
   // CTA pairs (2-CTA clusters) computing 256 x BN tiles with M = 256 MMAs.
   using Cfg2 = TcCfg<BN, 2>;
-  auto kern = tc_slice_gemm_kernel<BN, MODE, false, 2>;
-  if (!tc_regs_ok(reinterpret_cast<const void*>(kern))) return PHPC_ERR_UNSUPPORTED;
-  PHPC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg2::kSmem));
+  constexpr auto kern = tc_slice_gemm_kernel<BN, MODE, false, 2>;
+  if (const int rc = tc_ready<kern>(dev, Cfg2::kSmem); rc != PHPC_OK) return rc;
   cudaLaunchConfig_t cfg{};
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -259,10 +248,14 @@ int launch_tc_slice_gemm(const void* planesA, const void* planesB, int nplanesA,
   cfg.stream = stream;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cfg.gridDim = dim3(2 * static_cast<unsigned>(std::min<int64_t>(units, dev->sm_count / 2)), 1, 1);
-  int max_clusters = 0;
-  PHPC_CUDA_TRY(cudaOccupancyMaxActiveClusters(&max_clusters, kern, &cfg));
-  if (max_clusters < 1) return PHPC_ERR_UNSUPPORTED;
+  static PerDevice pairs_at_once;
+  int max_clusters = pairs_at_once.get(dev->ordinal);
+  if (max_clusters == 0) {
+    cfg.gridDim = dim3(2 * static_cast<unsigned>(dev->sm_count / 2), 1, 1);
+    PHPC_CUDA_TRY(cudaOccupancyMaxActiveClusters(&max_clusters, kern, &cfg));
+    if (max_clusters < 1) return PHPC_ERR_UNSUPPORTED;
+    pairs_at_once.set(dev->ordinal, max_clusters);
+  }
   cfg.gridDim = dim3(2 * static_cast<unsigned>(std::min<int64_t>(units, max_clusters)), 1, 1);
   PHPC_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, tmA, tmB, pairs, a, TcGroupTable{}));
   return PHPC_OK;

@@ -6,6 +6,7 @@
 #include <cudaTypedefs.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 #include <cstdio>
 
@@ -29,6 +30,17 @@ struct DeviceInfo {
   size_t smem_optin;
 };
 const DeviceInfo* current_device();
+
+// A value of 1 and up kept per device ordinal (a kernel attribute, an
+// occupancy): 0 until it is stored. Devices beyond the table are asked anew.
+struct PerDevice {
+  static constexpr int kDevices = 64;
+  std::atomic<int> v[kDevices] = {};
+  int get(int ordinal) const { return ordinal >= 0 && ordinal < kDevices ? v[ordinal].load(std::memory_order_acquire) : 0; }
+  void set(int ordinal, int value) {
+    if (ordinal >= 0 && ordinal < kDevices) v[ordinal].store(value, std::memory_order_release);
+  }
+};
 
 // cuTensorMapEncodeTiled, resolved once through cudaGetDriverEntryPointByVersion.
 bool encode_tiled(CUtensorMap* map, CUtensorMapDataType dtype, int rank, const void* base, const uint64_t* dims,

@@ -8,6 +8,7 @@
 #include <cmath>
 #include <cstdint>
 #include <cstdlib>
+#include <mutex>
 #include <type_traits>
 
 #include "crt.cuh"
@@ -62,13 +63,13 @@ inline int mod_crt_fast() {
   return (env && atoi(env) == 1) ? 0 : 1;
 }
 
-inline ModTable make_table(int nmod, int k) {
+// Everything but the worst-case width and the CRT path switch.
+inline ModTable make_moduli(int nmod) {
   using u128 = unsigned __int128;
   ModTable T{};
   T.n = nmod;
   u128 M = 1;
   for (int i = 0; i < nmod; ++i) M *= kModuli[i];
-  T.bits = mod_grid_bits(nmod, k);
   {
     double log_m = 0;
     for (int i = 0; i < nmod; ++i) log_m += std::log2(static_cast<double>(kModuli[i]));
@@ -110,7 +111,6 @@ inline ModTable make_table(int nmod, int k) {
   T.crt.qlimb = std::max(0, (bitlen - 51 + 31) / 32);
   T.crt.Minv = static_cast<float>(1.0 / static_cast<double>(static_cast<uint64_t>(M >> (32 * T.crt.qlimb))));
   T.crt.n = T.n;
-  T.crt.fast = mod_crt_fast();
   // the reconstruction on FP32 limbs: balanced 13-bit digits of M / m_i and M
   auto digits = [](u128 x, float2* out, int count) {
     int used = 0;
@@ -134,6 +134,18 @@ inline ModTable make_table(int nmod, int k) {
   float2 Md[kCrtMaxLimbs + 1];
   digits(M, Md, kCrtMaxLimbs + 1);
   for (int j = 0; j <= kCrtMaxLimbs; ++j) T.crt.L.negM[j] = make_float2(-Md[j].x, -Md[j].y);
+  return T;
+}
+
+// The constants of a modulus count never change: computed once, copied for
+// each call (computing them took about 5 us of host time, three times a call).
+inline ModTable make_table(int nmod, int k) {
+  static std::once_flag once[kMaxModuli + 1];
+  static ModTable tables[kMaxModuli + 1];
+  std::call_once(once[nmod], [&] { tables[nmod] = make_moduli(nmod); });
+  ModTable T = tables[nmod];
+  T.bits = mod_grid_bits(nmod, k);
+  T.crt.fast = mod_crt_fast();
   return T;
 }
 

@@ -44,6 +44,7 @@
 #pragma once
 #include "crt.cuh"
 #include "phpc_dev.cuh"
+#include "phpc_host.hpp"
 
 namespace phpc {
 
@@ -858,13 +859,25 @@ __global__ void __launch_bounds__(kTcThreads, 1)
 
 // The setmaxnreg split above redistributes exactly the registers the CTA was
 // launched with; it is only sound if the kernel was compiled with
-// kTcLaunchRegs registers per thread. Checked on the host before every launch
-// (a smaller count would make setmaxnreg.inc wait for registers that never
-// become free).
+// kTcLaunchRegs registers per thread. Checked on the host before a kernel's
+// first launch on a device (a smaller count would make setmaxnreg.inc wait
+// for registers that never become free).
 inline bool tc_regs_ok(const void* kernel) {
   cudaFuncAttributes fa;
   if (cudaFuncGetAttributes(&fa, kernel) != cudaSuccess) return false;
   return fa.numRegs == kTcLaunchRegs && fa.maxThreadsPerBlock >= kTcThreads;
+}
+
+// Kernel KERN is fit to launch on the device with smem bytes of dynamic
+// shared memory: the register check and the opt-in, once per device.
+template <auto KERN>
+int tc_ready(const DeviceInfo* dev, size_t smem) {
+  static PerDevice ready;
+  if (ready.get(dev->ordinal)) return PHPC_OK;
+  if (!tc_regs_ok(reinterpret_cast<const void*>(KERN))) return PHPC_ERR_UNSUPPORTED;
+  PHPC_CUDA_TRY(cudaFuncSetAttribute(KERN, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  ready.set(dev->ordinal, 1);
+  return PHPC_OK;
 }
 
 // Options of the host launcher below.
