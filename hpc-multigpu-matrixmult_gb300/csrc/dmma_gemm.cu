@@ -30,7 +30,6 @@ namespace phpc {
 namespace {
 
 constexpr int kBK = 16;         // doubles of K per stage (one 128-byte row of A)
-constexpr int kDefaultStages = 4;
 constexpr int kMaxStages = 6;   // ring depth bounds (PHPC_DMMA_STAGES, tuning table)
 
 struct SummaGrid {

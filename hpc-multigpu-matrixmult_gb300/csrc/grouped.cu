@@ -319,7 +319,7 @@ ProbLayout prob_layout(const phpc_gemm_problem& q, int planes, bool modular, boo
 }
 
 struct TableLayout {
-  size_t split, tprob, maps, tiles, sched, crt_first, rows_first, cols_prob, end;
+  size_t split, tprob, maps, tiles, sched, crt_first, rows_first, cols_prob, rmaps, end;
 };
 
 // Modular scheme: the lookup tables the plan writes for the CRT and the
@@ -360,7 +360,8 @@ LookupSizes lookup_sizes(const phpc_gemm_problem* problems, int count, bool modu
   return z;
 }
 
-TableLayout table_layout(int count, int64_t tiles, const LookupSizes& look) {
+// rmaps: with the residue planes' store maps (modular scheme).
+TableLayout table_layout(int count, int64_t tiles, const LookupSizes& look, bool rmaps) {
   TableLayout T;
   T.split = 0;
   T.tprob = align_up(sizeof(GSplitProb) * (size_t)count, 256);
@@ -370,7 +371,8 @@ TableLayout table_layout(int count, int64_t tiles, const LookupSizes& look) {
   T.crt_first = align_up(T.sched + sizeof(int), 256);  // modular scheme: the CRT blocks' first problems,
   T.rows_first = align_up(T.crt_first + sizeof(int) * (size_t)look.crt_blocks, 256);  // row blocks' first ones,
   T.cols_prob = align_up(T.rows_first + sizeof(int) * (size_t)look.row_blocks, 256);  // column blocks' problems
-  T.end = align_up(T.cols_prob + sizeof(int) * (size_t)look.col_blocks, 256);
+  T.rmaps = align_up(T.cols_prob + sizeof(int) * (size_t)look.col_blocks, 256);
+  T.end = align_up(T.rmaps + (rmaps ? sizeof(CUtensorMap) * (size_t)count : 0), 256);
   return T;
 }
 
@@ -444,7 +446,7 @@ int launch_grouped_gemm(const phpc_grouped_plan* pl, cudaStream_t stream) {
   if (pl->table.next_unit && cudaMemsetAsync(pl->table.next_unit, 0, sizeof(int), stream) != cudaSuccess)
     return PHPC_ERR_CUDA;
   const int grid = std::min(pl->total_tiles, dev->sm_count);
-  tc_slice_gemm_kernel<BN, MODE, true><<<grid, kTcThreads, Cfg::kSmem, stream>>>(dummy, dummy, pl->pairs, a,
+  tc_slice_gemm_kernel<BN, MODE, true><<<grid, kTcThreads, Cfg::kSmem, stream>>>(dummy, dummy, dummy, pl->pairs, a,
                                                                                  pl->table);
   return cudaGetLastError() == cudaSuccess ? PHPC_OK : PHPC_ERR_CUDA;
 }
@@ -510,9 +512,12 @@ int run_grouped(const phpc_grouped_plan* pl, cudaStream_t stream) {
   return rc;
 }
 
+// padded = false: the layout of a workspace without room for padded plane
+// rows and store maps.
 size_t grouped_workspace_bytes(const phpc_gemm_problem* problems, int count, int planes, bool modular,
                                bool padded = true) {
-  size_t total = table_layout(count, max_tiles(problems, count), lookup_sizes(problems, count, modular)).end;
+  size_t total =
+      table_layout(count, max_tiles(problems, count), lookup_sizes(problems, count, modular), modular && padded).end;
   for (int i = 0; i < count; ++i) {
     if (!valid_problem(problems[i])) return 0;
     total += prob_layout(problems[i], planes, modular, padded).end;
@@ -553,11 +558,12 @@ int grouped_plan_create(phpc_grouped_plan** out, const phpc_gemm_problem* proble
     pl->pairs = grouped_pairs(planes);
   }
 
-  const TableLayout T = table_layout(count, max_tiles(problems, count), lookup_sizes(problems, count, modular));
+  const TableLayout T = table_layout(count, max_tiles(problems, count), lookup_sizes(problems, count, modular),
+                                     modular && padded);
   uint8_t* base = static_cast<uint8_t*>(workspace);
   std::vector<GSplitProb> hs(count);
   std::vector<TcGroupProblem> ht(count);
-  std::vector<CUtensorMap> hm(2 * (size_t)count);
+  std::vector<CUtensorMap> hm(2 * (size_t)count), hmr(modular && padded ? count : 0);
   size_t off = T.end;
   int rows = 0, cols = 0, sblocks = 0, rblocks = 0, tiles = 0;
   int64_t pieces = 0, cunits = 0, crt_units = 0;
@@ -633,7 +639,8 @@ int grouped_plan_create(phpc_grouped_plan** out, const phpc_gemm_problem* proble
     const uint32_t bB[3] = {kTcBK, (uint32_t)pl->bn, 1};
     if (!encode_tiled(&hm[2 * i], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, g.pa, dA, sA, bA, CU_TENSOR_MAP_SWIZZLE_128B) ||
         !encode_tiled(&hm[2 * i + 1], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, g.pb, dB, sB, bB,
-                      CU_TENSOR_MAP_SWIZZLE_128B))
+                      CU_TENSOR_MAP_SWIZZLE_128B) ||
+        (!hmr.empty() && !encode_residue_planes(&hmr[i], g.R, q.m, q.n, planes, L.ldr, t.rplane)))
       rc = PHPC_ERR_CUDA;
     off += L.end;
   }
@@ -671,6 +678,7 @@ int grouped_plan_create(phpc_grouped_plan** out, const phpc_gemm_problem* proble
   pl->table.group_rows = 8;
   pl->table.probs = reinterpret_cast<const TcGroupProblem*>(base + T.tprob);
   pl->table.maps = reinterpret_cast<const CUtensorMap*>(base + T.maps);
+  pl->table.rmaps = hmr.empty() ? nullptr : reinterpret_cast<const CUtensorMap*>(base + T.rmaps);
   pl->table.tiles = reinterpret_cast<const int4*>(base + T.tiles);
   // units handed out in order by a counter (PHPC_GROUPED_SCHED=static: CTA c
   // takes units c, c + grid, ...)
@@ -700,6 +708,8 @@ int grouped_plan_create(phpc_grouped_plan** out, const phpc_gemm_problem* proble
            cudaSuccess ||
        cudaMemcpyAsync(base + T.maps, hm.data(), sizeof(CUtensorMap) * 2 * count, cudaMemcpyHostToDevice, st) !=
            cudaSuccess ||
+       (!hmr.empty() && cudaMemcpyAsync(base + T.rmaps, hmr.data(), sizeof(CUtensorMap) * hmr.size(),
+                                        cudaMemcpyHostToDevice, st) != cudaSuccess) ||
        (tiles > 0 && cudaMemcpyAsync(base + T.tiles, htiles.data(), sizeof(int4) * tiles, cudaMemcpyHostToDevice,
                                      st) != cudaSuccess) ||
        (!hfirst.empty() && cudaMemcpyAsync(base + T.crt_first, hfirst.data(), sizeof(int) * hfirst.size(),

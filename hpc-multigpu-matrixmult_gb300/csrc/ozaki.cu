@@ -25,6 +25,7 @@
 // ~2000x below its BF16 tensor rate.
 #include <algorithm>
 #include <cstdlib>
+#include <cstring>
 #include <mutex>
 
 #include <cuda_bf16.h>
@@ -180,6 +181,9 @@ int launch_tc_slice_gemm(const void* planesA, const void* planesB, int nplanesA,
   if (!encode_tiled(&tmA, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, planesA, dA, sA, bA, CU_TENSOR_MAP_SWIZZLE_128B) ||
       !encode_tiled(&tmB, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, planesB, dB, sB, bB, CU_TENSOR_MAP_SWIZZLE_128B))
     return PHPC_ERR_CUDA;
+  CUtensorMap tmR;
+  std::memset(&tmR, 0, sizeof tmR);
+  if (MODE == kResidue && !encode_residue_planes(&tmR, R, m, n, pairs.n, ldr, rplane)) return PHPC_ERR_CUDA;
   TcArgs a{};
   a.M = m;
   a.N = n;
@@ -221,7 +225,7 @@ int launch_tc_slice_gemm(const void* planesA, const void* planesB, int nplanesA,
       cudaLaunchConfig_t cfg = ksplit_config<BN>(a.ksplit, attr);
       cfg.gridDim = dim3(static_cast<unsigned>(a.tm * a.tn * a.ksplit), 1, 1);
       cfg.stream = stream;
-      PHPC_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, tmA, tmB, pairs, a, TcGroupTable{}));
+      PHPC_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, tmA, tmB, tmR, pairs, a, TcGroupTable{}));
       return PHPC_OK;
     }
   }
@@ -229,7 +233,7 @@ int launch_tc_slice_gemm(const void* planesA, const void* planesB, int nplanesA,
     constexpr auto kern = tc_slice_gemm_kernel<BN, MODE>;
     if (const int rc = tc_ready<kern>(dev, Cfg::kSmem); rc != PHPC_OK) return rc;
     const int grid = static_cast<int>(std::min<int64_t>(units, dev->sm_count));
-    kern<<<grid, kTcThreads, Cfg::kSmem, stream>>>(tmA, tmB, pairs, a, TcGroupTable{});
+    kern<<<grid, kTcThreads, Cfg::kSmem, stream>>>(tmA, tmB, tmR, pairs, a, TcGroupTable{});
     PHPC_CUDA_TRY(cudaGetLastError());
     return PHPC_OK;
   }
@@ -257,7 +261,7 @@ int launch_tc_slice_gemm(const void* planesA, const void* planesB, int nplanesA,
     pairs_at_once.set(dev->ordinal, max_clusters);
   }
   cfg.gridDim = dim3(2 * static_cast<unsigned>(std::min<int64_t>(units, max_clusters)), 1, 1);
-  PHPC_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, tmA, tmB, pairs, a, TcGroupTable{}));
+  PHPC_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, tmA, tmB, tmR, pairs, a, TcGroupTable{}));
   return PHPC_OK;
 }
 

@@ -18,8 +18,8 @@
 //          that stays an exact integer; at the end of the modulus the sum is
 //          stored as one 16-bit residue per element in residue plane i of R,
 //          and the CRT pass (ozaki2.cu) combines the planes. Residues leave
-//          through the warp's scratch so that each store instruction writes
-//          four 128-byte row segments. The moduli are independent: with
+//          through the warp's scratch by TMA stores of 32 rows x 64 columns.
+//          The moduli are independent: with
 //          split_pairs a work unit is one (tile, modulus), moduli outer, so
 //          that consecutive waves of CTAs share one modulus's planes in L2
 //          and a ragged last wave is spread over more units; every other
@@ -135,6 +135,8 @@ struct TcGroupTable {
   int group_rows;
   const TcGroupProblem* probs;  // [count]
   const CUtensorMap* maps;      // [2 * count], 64-byte aligned
+  const CUtensorMap* rmaps;     // kResidue: [count], the residue planes (stores), or nullptr (a plan in a
+                                // workspace without room for them: the epilogue stores from registers)
   const int4* tiles;            // [ntiles]: (problem, tile row, tile column, K-steps), one load per tile
   int* next_unit;               // non-null: units handed out in order by this counter (zeroed before
                                 // each launch), else CTA c takes units c, c + grid, ...
@@ -155,6 +157,7 @@ struct TcJob {
   int M, N, nk, rm, rn;
   const CUtensorMap* tmA;
   const CUtensorMap* tmB;
+  const CUtensorMap* tmR;
   void* C;
   int64_t ldc;
   const int* ea;
@@ -174,7 +177,8 @@ struct TcCfg {
   static constexpr int kStageB = (BN / CLUSTER) * kTcBK * 2;
   static constexpr int kStageBytes = kStageA + kStageB;
   static constexpr int kStages = (192 * 1024) / kStageBytes;  // 4 / 6 (BN 256, solo / pair), 6 / 8 (BN 128)
-  static constexpr int kScratchPerWarp = 32 * 33 * 4;       // 32x32 transpose tile, padded
+  static constexpr int kScratchPerWarp = 32 * 33 * 4;       // 32x32 transpose tile, padded (kResidue: 4 KB, a
+                                                            // 32 x 64 store box)
   static constexpr int kTmemCols = 2 * BN;                  // two accumulator buffers
   static constexpr size_t kSmem =
       (size_t)kStages * kStageBytes + kTcEpiWarps * kScratchPerWarp + 512 /*barriers, unit queue*/ + 1024 /*align*/;
@@ -198,7 +202,7 @@ __host__ __device__ __forceinline__ void tc_tile_coords(int tm, int tn, int grou
 // nothing).
 template <bool GROUPED, int CLUSTER>
 __device__ __forceinline__ void tc_job(int t, const TcArgs& a, const CUtensorMap* tmA, const CUtensorMap* tmB,
-                                       const TcGroupTable& g, uint32_t crank, TcJob& j) {
+                                       const CUtensorMap* tmR, const TcGroupTable& g, uint32_t crank, TcJob& j) {
   if (!GROUPED) {
     j.M = a.M;
     j.N = a.N;
@@ -212,6 +216,7 @@ __device__ __forceinline__ void tc_job(int t, const TcArgs& a, const CUtensorMap
     }
     j.tmA = tmA;
     j.tmB = tmB;
+    j.tmR = tmR;
     j.C = a.C;
     j.ldc = a.ldc;
     j.ea = a.ea;
@@ -232,6 +237,7 @@ __device__ __forceinline__ void tc_job(int t, const TcArgs& a, const CUtensorMap
     j.rn = e.z;
     j.tmA = g.maps + 2 * lo;
     j.tmB = g.maps + 2 * lo + 1;
+    j.tmR = g.rmaps ? g.rmaps + lo : nullptr;
     j.C = p.C;
     j.ldc = p.ldc;
     j.ea = p.ea;
@@ -272,7 +278,7 @@ __device__ __forceinline__ uint32_t ksplit_chunk(int r, int c) {
 template <int BN, int MODE, bool GROUPED = false, int CLUSTER = 1, bool KSPLIT = false>
 __global__ void __launch_bounds__(kTcThreads, 1)
     tc_slice_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                         const __grid_constant__ PairList pairs, const __grid_constant__ TcArgs args,
+                         const __grid_constant__ CUtensorMap tmR, const __grid_constant__ PairList pairs, const __grid_constant__ TcArgs args,
                          const __grid_constant__ TcGroupTable gt) {
   static_assert(CLUSTER == 1 || (CLUSTER == 2 && !GROUPED), "the CTA pair computes tiles of one problem");
   static_assert(!KSPLIT || (MODE == kF32 && CLUSTER == 1 && !GROUPED), "K is split in the FP32 GEMM only");
@@ -393,7 +399,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
           u = u_ahead < nunits ? u_ahead : -1;
           if (u >= 0) {
             tc_unit(u, ntiles, split, t, p0);
-            tc_job<GROUPED, CLUSTER>(t, args, &tmA, &tmB, gt, crank, job);
+            tc_job<GROUPED, CLUSTER>(t, args, &tmA, &tmB, &tmR, gt, crank, job);
           }
           // the MMA issuer gets the unit's K-steps with it (no table lookups on its path)
           uq_unit[q] = make_int2(u, u >= 0 ? job.nk : 0);
@@ -405,7 +411,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
           u = unit0 + i * ustride;
           if (u >= nunits) break;
           tc_unit(u, ntiles, split, t, p0);
-          tc_job<GROUPED, CLUSTER>(t, args, &tmA, &tmB, gt, crank, job);
+          tc_job<GROUPED, CLUSTER>(t, args, &tmA, &tmB, &tmR, gt, crank, job);
         }
         const int p1 = split ? p0 + 1 : pairs.n;
         const bool rev = serp && (round & 1);
@@ -476,7 +482,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         const int p1 = split ? p0 + 1 : pairs.n;
         if (!dyn) {
           TcJob job;
-          tc_job<GROUPED, CLUSTER>(t, args, &tmA, &tmB, gt, crank, job);
+          tc_job<GROUPED, CLUSTER>(t, args, &tmA, &tmB, &tmR, gt, crank, job);
           nk = job.nk;
         }
         int gstart = p0;
@@ -574,7 +580,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       tc_unit(u, ntiles, split, t, p0);
       const int p1 = split ? p0 + 1 : pairs.n;
       TcJob job;
-      tc_job<GROUPED, CLUSTER>(t, args, &tmA, &tmB, gt, crank, job);
+      tc_job<GROUPED, CLUSTER>(t, args, &tmA, &tmB, &tmR, gt, crank, job);
       const int64_t row0 = (int64_t)job.rm * kTcBM + quad * 32;  // first global row of this warp's quadrant
       const int col0 = job.rn * BN + half * HALF;                 // first global column of this warp's half
       int my_ea = 0;
@@ -677,28 +683,44 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             }
             // One 16-bit value per element, 64 columns at a time: each lane
             // writes its row's 64 values into the warp's scratch as eight
-            // 16-byte chunks (row r's chunk c at position c ^ (r % 8), so
-            // that the 8 lanes of a quarter-warp hit distinct banks), then
-            // the warp stores 4 rows x 128 bytes per instruction (lane: row
-            // 4 i + lane / 8, 16-byte segment lane % 8), reading its chunk
-            // with one 16-byte load. (acc holds exact f32 integers: the chunk
-            // itself, or the sum of the reduced chunks.)
-            uint16_t* rplane = job.R + static_cast<int64_t>(pairs.g[gstart]) * job.rplane;
-            uint4* tq = reinterpret_cast<uint4*>(tr);  // [32 rows][8 chunks], 4 KB of the warp's scratch
+            // 16-byte chunks (row r's chunk c at position c ^ (r % 8), the
+            // 128-byte swizzle, so that the 8 lanes of a quarter-warp hit
+            // distinct banks), and one TMA store takes the 32 x 64 box to the
+            // residue plane (rows and columns beyond the matrix clipped). The
+            // values are formed before the wait for the last box's read. (acc
+            // holds exact f32 integers: the chunk itself, or the sum of the
+            // reduced chunks.) Stores from registers, 4 rows x 128 bytes an
+            // instruction, set the pace of units of few K-steps: N = 4096, K =
+            // 512 184 us against 170, K = 128 115 against 87 (128 and 52
+            // without any stores or arithmetic).
+            const int plane = pairs.g[gstart];
+            uint4* tq = reinterpret_cast<uint4*>(scratch + ew * 4096);  // [32 rows][8 chunks]
 #pragma unroll
             for (int h = 0; h < HALF; h += 64) {
+              uint32_t w[32];
 #pragma unroll
-              for (int c = 0; c < 8; ++c) {
-                uint32_t w[4];
-#pragma unroll
-                for (int e = 0; e < 4; ++e)
-                  w[e] = crt_t_pair(__int_as_float(acc[h + 8 * c + 2 * e]), __int_as_float(acc[h + 8 * c + 2 * e + 1]),
-                                        mf, invm);
-                tq[lane * 8 + (c ^ (lane & 7))] = make_uint4(w[0], w[1], w[2], w[3]);
-              }
+              for (int e = 0; e < 32; ++e)
+                w[e] = crt_t_pair(__int_as_float(acc[h + 2 * e]), __int_as_float(acc[h + 2 * e + 1]), mf, invm);
+              if (lane == 0) bulk_wait_read();
               __syncwarp();
+#pragma unroll
+              for (int c = 0; c < 8; ++c)
+                tq[lane * 8 + (c ^ (lane & 7))] = make_uint4(w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
+              const int colh = col0 + h;
+              if (!GROUPED || job.tmR != nullptr) {
+                fence_proxy_async();
+                __syncwarp();
+                if (lane == 0 && row0 < job.M && colh < job.N) {
+                  tma_store_3d(job.tmR, tq, colh, static_cast<int>(row0), plane);
+                  bulk_commit();
+                }
+                continue;
+              }
+              // a grouped plan without store maps
+              __syncwarp();
+              uint16_t* rplane = job.R + static_cast<int64_t>(plane) * job.rplane;
               const int seg = lane & 7;
-              const int col = col0 + h + seg * 8;
+              const int col = colh + seg * 8;
 #pragma unroll
               for (int i = 0; i < 8; ++i) {
                 const int r = 4 * i + (lane >> 3);
@@ -789,10 +811,11 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         gstart = gend;
       }
     }
+    if (MODE == kResidue && lane == 0) bulk_wait_all();  // the stores have left shared memory
     if (KSPLIT) {
       cluster_sync();  // every CTA's sums are in its shared memory
       TcJob job;
-      tc_job<GROUPED, CLUSTER>(unit0, args, &tmA, &tmB, gt, crank, job);
+      tc_job<GROUPED, CLUSTER>(unit0, args, &tmA, &tmB, &tmR, gt, crank, job);
       const uint32_t base = smem_u32(smem);
       // this CTA's rows, four 16-byte chunks a thread at a time, four CTAs' sums
       // of each in flight, their C values on the way meanwhile
@@ -878,6 +901,16 @@ int tc_ready(const DeviceInfo* dev, size_t smem) {
   PHPC_CUDA_TRY(cudaFuncSetAttribute(KERN, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
   ready.set(dev->ordinal, 1);
   return PHPC_OK;
+}
+
+// Map of the residue planes R [q][.][ldr] for the epilogue's stores: boxes of
+// 32 rows x 64 columns (128 bytes, swizzled).
+inline bool encode_residue_planes(CUtensorMap* map, const uint16_t* R, int m, int n, int q, int64_t ldr,
+                                  int64_t rplane) {
+  const uint64_t d[3] = {(uint64_t)n, (uint64_t)m, (uint64_t)q};
+  const uint64_t s[2] = {(uint64_t)ldr * 2, (uint64_t)rplane * 2};
+  const uint32_t b[3] = {64, 32, 1};
+  return encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_UINT16, 3, R, d, s, b, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
 // Options of the host launcher below.
