@@ -153,14 +153,37 @@ int default_bn(int m, int k, int n) {
   return 256;
 }
 
+namespace {
+
+// Whether CTA pairs suit the shape where the table has them. A pair stages 32
+// KB a K-step and SM against 48, but its units cost more to start and to drain:
+//  - fewer than 80 K-steps an SM (residue GEMM, 13 moduli): N = 1024 25.5 us
+//    single, 29.0 in pairs; 1024 x 2048 x 1024 49.1, 47.4; 2048 x 512 x 2048
+//    51.9, 48.2;
+//  - a last accumulator chunk (of 8 K-steps) that is half empty or emptier, or
+//    a single short one, leaves the MMAs waiting for the drain of the pair's
+//    other chunk: 4096 x K x 4096 with K = 256 110, 148; 384 144, 145; 512
+//    171, 156; 520 208, 235; 700 227, 244; 830 258, 256; 1000 318, 285; 1100
+//    344, 362; 2000 548, 526;
+//  - an odd number of tile rows pads the last pair: 1400 (11 rows) 63.9, 70.1;
+//    600 x 4096 x 2000 (5) 109, 121; 1537 x 1000 x 2311 (13) 86.5, 84.3.
+bool pairs_fit(int m, int k, int n) {
+  const int64_t rows = ceil_div(m, 128), steps = ceil_div(k, 64), units = (rows + 1) / 2 * ceil_div(n, 256) * 13;
+  const bool full = steps % 8 == 0 || steps % 8 > 4 || steps > 32;
+  return full && steps >= 8 && units * steps >= 80 * 76 && (rows % 2 == 0 || rows > 12);
+}
+
+}  // namespace
+
 // CTAs per cluster of the single-problem slice GEMM (1, or 2 = a CTA pair
 // computing one 256-row tile with cta_group::2 MMAs, each CTA loading its own
-// half of the operands): PHPC_CLUSTER, else the table, else 1.
+// half of the operands): PHPC_CLUSTER, else the table's choice where pairs
+// suit the shape, else 1.
 int default_cluster(int m, int k, int n) {
   const char* env = getenv("PHPC_CLUSTER");
   if (env && (atoi(env) == 1 || atoi(env) == 2)) return atoi(env);
   if (const TuneEntry* e = lookup(m, k, n))
-    if (e->cluster == 2) return 2;
+    if (e->cluster == 2 && pairs_fit(m, k, n)) return 2;
   return 1;
 }
 
