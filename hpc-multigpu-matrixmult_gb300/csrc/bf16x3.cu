@@ -35,36 +35,45 @@ __device__ __forceinline__ void split3(float x, uint16_t& h1, uint16_t& h2, uint
   h3 = __bfloat16_as_ushort(b3);
 }
 
-// A: plane p holds slice p of A[i][k] at [p][i][k]; 8 consecutive k per thread.
-__global__ void split3_rows_kernel(const float* __restrict__ A, int64_t lda, int M, int K,
-                                   uint16_t* __restrict__ planes, int64_t ldp, int64_t plane_stride) {
-  const int64_t row = blockIdx.x;
-  const int64_t k0 = ((int64_t)blockIdx.y * blockDim.x + threadIdx.x) * 8;
-  if (row >= M || k0 >= K) return;
-  const float* a = A + row * lda;
-  uint32_t w[3][4];
-#pragma unroll
-  for (int j = 0; j < 8; j += 2) {
-    uint16_t x0[3], x1[3];
-    split3(k0 + j < K ? a[k0 + j] : 0.f, x0[0], x0[1], x0[2]);
-    split3(k0 + j + 1 < K ? a[k0 + j + 1] : 0.f, x1[0], x1[1], x1[2]);
-#pragma unroll
-    for (int p = 0; p < 3; ++p) w[p][j >> 1] = (uint32_t)x0[p] | ((uint32_t)x1[p] << 16);
-  }
-#pragma unroll
-  for (int p = 0; p < 3; ++p)
-    *reinterpret_cast<uint4*>(planes + p * plane_stride + row * ldp + k0) = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
-}
+constexpr int kSplit3Threads = 256;
 
-// B, transposed: plane p holds slice p of B[k][j] at [p][j][k]; 32 (k) x 64 (j) per CTA.
-__global__ void __launch_bounds__(256) split3_cols_kernel(const float* __restrict__ B, int64_t ldb, int K, int N,
-                                                          uint16_t* __restrict__ planes, int64_t ldp,
-                                                          int64_t plane_stride) {
+// Both operands in one launch, A's blocks first. A: plane p holds slice p of
+// A[i][k] at [p][i][k]; 8 consecutive k (a piece) per thread, pieces numbered
+// row by row. B, transposed: plane p holds slice p of B[k][j] at [p][j][k]; 32
+// (k) x 64 (j) per block. (Two launches one after the other took 4 + 6 us of a
+// 1000 x 777 x 1530 call.)
+__global__ void __launch_bounds__(kSplit3Threads)
+    split3_kernel(const float* __restrict__ A, int64_t lda, int M, const float* __restrict__ B, int64_t ldb, int N,
+                  int K, uint16_t* __restrict__ pa, uint16_t* __restrict__ pb, int64_t ldp, int64_t a_blocks,
+                  int strips) {
   __shared__ uint32_t st[3][64][17];
+  pdl_trigger();
+  if (blockIdx.x < a_blocks) {
+    const int per_row = (K + 7) >> 3;
+    const int64_t t = (int64_t)blockIdx.x * kSplit3Threads + threadIdx.x, pieces = (int64_t)M * per_row;
+    if (t >= pieces) return;
+    const int64_t row = pieces <= UINT32_MAX ? static_cast<uint32_t>(t) / static_cast<uint32_t>(per_row) : t / per_row;
+    const int64_t k0 = (t - row * per_row) * 8, plane = (int64_t)M * ldp;
+    const float* a = A + row * lda;
+    uint32_t w[3][4];
+#pragma unroll
+    for (int j = 0; j < 8; j += 2) {
+      uint16_t x0[3], x1[3];
+      split3(k0 + j < K ? a[k0 + j] : 0.f, x0[0], x0[1], x0[2]);
+      split3(k0 + j + 1 < K ? a[k0 + j + 1] : 0.f, x1[0], x1[1], x1[2]);
+#pragma unroll
+      for (int p = 0; p < 3; ++p) w[p][j >> 1] = (uint32_t)x0[p] | ((uint32_t)x1[p] << 16);
+    }
+#pragma unroll
+    for (int p = 0; p < 3; ++p)
+      *reinterpret_cast<uint4*>(pa + p * plane + row * ldp + k0) = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
+    return;
+  }
+  const int64_t blk = blockIdx.x - a_blocks;
   const int j = threadIdx.x & 63;
   const int kp0 = threadIdx.x >> 6;
-  const int64_t k0 = (int64_t)blockIdx.y * 32;
-  const int64_t j0 = (int64_t)blockIdx.x * 64;
+  const int64_t k0 = blk / strips * 32;
+  const int64_t j0 = blk % strips * 64;
   const int64_t col = j0 + j;
   for (int kp = kp0; kp < 16; kp += 4) {
     const int64_t k = k0 + 2 * kp;
@@ -80,7 +89,7 @@ __global__ void __launch_bounds__(256) split3_cols_kernel(const float* __restric
   if (gj >= N || gk >= K) return;
 #pragma unroll
   for (int p = 0; p < 3; ++p)
-    *reinterpret_cast<uint4*>(planes + p * plane_stride + gj * ldp + gk) =
+    *reinterpret_cast<uint4*>(pb + p * ((int64_t)N * ldp) + gj * ldp + gk) =
         make_uint4(st[p][wj][4 * q], st[p][wj][4 * q + 1], st[p][wj][4 * q + 2], st[p][wj][4 * q + 3]);
 }
 
@@ -223,22 +232,26 @@ extern "C" int phpc_sgemm_bf16x3_dev(int m, int k, int n, const float* dA, int64
       rc = PHPC_ERR_UNSUPPORTED;
     } else if (!workspace || workspace_bytes < L.total || !aligned16(workspace)) {
       rc = PHPC_ERR_WORKSPACE;
+    } else if (ceil_div(k, 32) > 65535) {
+      rc = PHPC_ERR_CUDA;  // K beyond what the split has ever taken
     } else {
       uint16_t* pa = reinterpret_cast<uint16_t*>(static_cast<uint8_t*>(workspace) + L.off_pa);
       uint16_t* pb = reinterpret_cast<uint16_t*>(static_cast<uint8_t*>(workspace) + L.off_pb);
-      split3_rows_kernel<<<dim3(m, ceil_div(k, 8 * 128)), 128, 0, st>>>(dA, lda, m, k, pa, L.ldp,
-                                                                            (int64_t)m * L.ldp);
-      split3_cols_kernel<<<dim3(ceil_div(n, 64), ceil_div(k, 32)), 256, 0, st>>>(dB, ldb, k, n, pb, L.ldp,
-                                                                                 (int64_t)n * L.ldp);
+      const int64_t a_blocks = ((int64_t)m * ceil_div(k, 8) + kSplit3Threads - 1) / kSplit3Threads;
+      const int strips = ceil_div(n, 64);
+      split3_kernel<<<static_cast<unsigned>(a_blocks + (int64_t)strips * ceil_div(k, 32)), kSplit3Threads, 0, st>>>(
+          dA, lda, m, dB, ldb, n, k, pa, pb, L.ldp, a_blocks, strips);
       if (cudaGetLastError() != cudaSuccess) {
         rc = PHPC_ERR_CUDA;
       } else {
         const PairList pl = bf16x3_pairs();
+        TcGemmOpts opt;
+        opt.dependent = true;
         rc = default_f32(m, k, n).bn == 128
                  ? launch_tc_slice_gemm<128, kF32>(pa, pb, 3, 3, L.ldp, m, n, k, pl, dC, ldc, nullptr, nullptr, st,
-                                                   nullptr, 0, 0)
+                                                   nullptr, 0, 0, opt)
                  : launch_tc_slice_gemm<256, kF32>(pa, pb, 3, 3, L.ldp, m, n, k, pl, dC, ldc, nullptr, nullptr, st,
-                                                   nullptr, 0, 0);
+                                                   nullptr, 0, 0, opt);
       }
     }
   }

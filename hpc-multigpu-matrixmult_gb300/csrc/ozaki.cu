@@ -95,6 +95,13 @@ PairList ozaki_pairs(int s) {
 
 namespace {
 
+// Adds the attribute of a dependent launch (launch_dependent) to a config's list.
+void dependent_attr(cudaLaunchAttribute* attr, cudaLaunchConfig_t& cfg) {
+  attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
+  ++cfg.numAttrs;
+}
+
 template <int BN>
 cudaLaunchConfig_t ksplit_config(int split, cudaLaunchAttribute* attr) {
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -216,13 +223,15 @@ int launch_tc_slice_gemm(const void* planesA, const void* planesB, int nplanesA,
   }
   const int64_t units =
       (cluster == 1 ? (int64_t)a.tm * a.tn : (int64_t)((a.tm + 1) / 2) * a.tn) * (a.split_pairs ? pairs.n : 1);
+  const bool dependent = opt.dependent && short_gemm(m, n, pairs.n * ceil_div(k, kTcBK), dev->sm_count);
   if constexpr (MODE == kF32) {
     a.ksplit = f32_ksplit<BN>(m, n, pairs.n * ceil_div(k, kTcBK), dev);
     if (a.ksplit > 1) {
       constexpr auto kern = tc_slice_gemm_kernel<BN, MODE, false, 1, true>;
       if (const int rc = tc_ready<kern>(dev, Cfg::kSmem); rc != PHPC_OK) return rc;
-      cudaLaunchAttribute attr[1];
+      cudaLaunchAttribute attr[2];
       cudaLaunchConfig_t cfg = ksplit_config<BN>(a.ksplit, attr);
+      if (dependent) dependent_attr(attr, cfg);
       cfg.gridDim = dim3(static_cast<unsigned>(a.tm * a.tn * a.ksplit), 1, 1);
       cfg.stream = stream;
       PHPC_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, tmA, tmB, tmR, pairs, a, TcGroupTable{}));
@@ -233,8 +242,8 @@ int launch_tc_slice_gemm(const void* planesA, const void* planesB, int nplanesA,
     constexpr auto kern = tc_slice_gemm_kernel<BN, MODE>;
     if (const int rc = tc_ready<kern>(dev, Cfg::kSmem); rc != PHPC_OK) return rc;
     const int grid = static_cast<int>(std::min<int64_t>(units, dev->sm_count));
-    kern<<<grid, kTcThreads, Cfg::kSmem, stream>>>(tmA, tmB, tmR, pairs, a, TcGroupTable{});
-    PHPC_CUDA_TRY(cudaGetLastError());
+    PHPC_CUDA_TRY(launch_dependent(dependent, kern, grid, kTcThreads, Cfg::kSmem, stream, tmA, tmB, tmR, pairs, a,
+                                   TcGroupTable{}));
     return PHPC_OK;
   }
   // CTA pairs (2-CTA clusters) computing 256 x BN tiles with M = 256 MMAs.
@@ -242,7 +251,7 @@ int launch_tc_slice_gemm(const void* planesA, const void* planesB, int nplanesA,
   constexpr auto kern = tc_slice_gemm_kernel<BN, MODE, false, 2>;
   if (const int rc = tc_ready<kern>(dev, Cfg2::kSmem); rc != PHPC_OK) return rc;
   cudaLaunchConfig_t cfg{};
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = 1;
@@ -261,6 +270,7 @@ int launch_tc_slice_gemm(const void* planesA, const void* planesB, int nplanesA,
     pairs_at_once.set(dev->ordinal, max_clusters);
   }
   cfg.gridDim = dim3(2 * static_cast<unsigned>(std::min<int64_t>(units, max_clusters)), 1, 1);
+  if (dependent) dependent_attr(attr, cfg);
   PHPC_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, tmA, tmB, tmR, pairs, a, TcGroupTable{}));
   return PHPC_OK;
 }

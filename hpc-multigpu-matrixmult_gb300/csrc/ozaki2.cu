@@ -81,6 +81,7 @@ __global__ void __launch_bounds__(kPrepThreads) scan_kernel(const PrepRows a, co
   __shared__ int se[8][32];
   __shared__ float ss[8][32];
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  pdl_trigger();
   NormAcc acc;
   bool nf = false;
   if (static_cast<int>(blockIdx.x) < row_blocks) {
@@ -122,6 +123,8 @@ __global__ void __launch_bounds__(256) scan_cols_merge_kernel(int K, int N, int6
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
   const int64_t col = (int64_t)blockIdx.x * 32 + l;
   const int chunks = (K + kNormChunk - 1) / kNormChunk;
+  pdl_trigger();
+  pdl_wait();
   NormAcc acc = norm_merge_strided(pe, ps, ldpart, col, col < N ? chunks : 0, w);
   se[w][l] = acc.e;
   ss[w][l] = acc.s;
@@ -156,6 +159,8 @@ __global__ void __launch_bounds__(kPrepThreads, 4)
     residue_split_kernel(const PrepRows a, const PrepCols b, int row_blocks, int strips, int K, int64_t ldp,
                          const __grid_constant__ ModTable T) {
   __shared__ double tile[kColBlockK][kColBlockJ];
+  pdl_trigger();
+  pdl_wait();
   if (static_cast<int>(blockIdx.x) < row_blocks) {
     const int per_row = (K + 7) >> 3, ranges = per_row / kPrepThreads, left = per_row - ranges * kPrepThreads;
     const int64_t blk = blockIdx.x, full = (int64_t)a.rows * ranges;
@@ -202,6 +207,7 @@ __global__ void __launch_bounds__(128, crt_min_blocks(NMOD, false))
                const __grid_constant__ ModTable T, double* __restrict__ C, int64_t ldc) {
   const int64_t row = blockIdx.x;
   const int64_t c0 = ((int64_t)blockIdx.y * blockDim.x + threadIdx.x) * kCrtCols;
+  pdl_wait();
   if (row >= M || c0 >= N) return;
   crt_cols<NMOD>(R + row * ldr + c0, rplane, T.crt, T.crt.fast, static_cast<int>(min(static_cast<int64_t>(kCrtCols), N - c0)),
            max(ea[row], -20000) - ba[row], eb + c0, bb + c0, C + row * ldc + c0);
@@ -284,16 +290,19 @@ int prepare_operands(const PrepRows& a, PrepCols b, int k, int64_t ldp, const Mo
   const int ranges = ceil_div(k, 8) / kPrepThreads, left = ceil_div(k, 8) - ranges * kPrepThreads;
   const int split_rows = a.rows * ranges + ceil_div((int64_t)a.rows * left, kPrepThreads);
   b.merge = chunks <= kMergeInSplit;
+  const bool both = a.rows > 0 && b.cols > 0;  // one side: another stream's kernels share the SMs
   scan_kernel<<<scan_rows + strips * chunks, kPrepThreads, 0, stream>>>(a, b, scan_rows, strips, k, T.logT,
                                                                         device_status_ptr());
-  if (b.cols > 0 && !b.merge)
-    scan_cols_merge_kernel<<<strips, 256, 0, stream>>>(k, b.cols, b.ldpart, b.pe, b.ps, b.eb, b.bb, T.logT);
-  with_crt_moduli(T.n, [&](auto nm) {
-    residue_split_kernel<decltype(nm)::value>
-        <<<split_rows + strips * ceil_div(k, kColBlockK), kPrepThreads, 0, stream>>>(a, b, split_rows, strips, k, ldp,
-                                                                                     T);
-  });
   PHPC_CUDA_TRY(cudaGetLastError());
+  if (b.cols > 0 && !b.merge)
+    PHPC_CUDA_TRY(launch_dependent(both, scan_cols_merge_kernel, strips, 256, 0, stream, k, b.cols, b.ldpart, b.pe,
+                                   b.ps, b.eb, b.bb, T.logT));
+  cudaError_t e = cudaSuccess;
+  with_crt_moduli(T.n, [&](auto nm) {
+    e = launch_dependent(both, residue_split_kernel<decltype(nm)::value>, split_rows + strips * ceil_div(k, kColBlockK),
+                         kPrepThreads, 0, stream, a, b, split_rows, strips, k, ldp, T);
+  });
+  PHPC_CUDA_TRY(e);
   return PHPC_OK;
 }
 static_assert(kColBlockJ == 32, "scan strips are the split's column blocks");
@@ -357,8 +366,11 @@ int ozaki2_prepare2(int m, int k, int n, const double* dA, int64_t lda, const do
 // B's scans and split run on this thread's side stream beside A's (both are
 // memory-bound; run together, one's ramp-up and tail overlap the other's), and
 // the caller's stream waits for them.
+// *joined: whether another stream's work joined it (then the next launch does
+// not directly follow a kernel).
 int ozaki2_prepare_on(int m, int k, int n, const double* dA, int64_t lda, const double* dB, int64_t ldb, int nmod,
-                      void* ws, size_t ws_bytes, cudaStream_t stream) {
+                      void* ws, size_t ws_bytes, cudaStream_t stream, bool* joined = nullptr) {
+  if (joined) *joined = false;
   if (ceil_div(k, kNormChunk) <= kMergeInSplit && ((int64_t)m + n) * k < (4 << 20)) {
     Ozaki2Layout L;
     Ozaki2Views V;
@@ -369,6 +381,7 @@ int ozaki2_prepare_on(int m, int k, int n, const double* dA, int64_t lda, const 
   }
   const cudaStream_t side = side_stream();
   if (!side || !stream_fork(stream, side)) return ozaki2_prepare2(m, k, n, dA, lda, dB, ldb, nmod, ws, ws_bytes, stream, stream);
+  if (joined) *joined = true;
   int rc = ozaki2_prepare2(m, k, n, dA, lda, dB, ldb, nmod, ws, ws_bytes, stream, side);
   if (!stream_fork(side, stream) && rc == PHPC_OK) rc = PHPC_ERR_CUDA;
   return rc;
@@ -378,7 +391,7 @@ int ozaki2_prepare_on(int m, int k, int n, const double* dA, int64_t lda, const 
 // cols): plane i of R = (A_i * B_i^T) mod m_i, one 16-bit residue per element.
 // Tile width, cluster and raster are those of the full m x k x n problem.
 int ozaki2_multiply_block(int m, int r0, int rows, int c0, int cols, int k, int n, int nmod, const void* ws,
-                          size_t ws_bytes, cudaStream_t stream, int bn) {
+                          size_t ws_bytes, cudaStream_t stream, int bn, bool dependent) {
   Ozaki2Layout L;
   Ozaki2Views V;
   const int rc = ozaki2_views(m, k, n, nmod, ws, ws_bytes, L, V);
@@ -404,6 +417,7 @@ int ozaki2_multiply_block(int m, int r0, int rows, int c0, int cols, int k, int 
   opt.cfg_m = m;
   opt.cfg_n = n;
   opt.cfg_k = k;
+  opt.dependent = dependent;
   return bn == 128 ? launch_tc_slice_gemm<128, kResidue>(pa, pb, nmod, nmod, L.ldp, rows, cols, k, pl, nullptr, 0,
                                                           nullptr, nullptr, stream, R, L.ldr, rplane, opt)
                    : launch_tc_slice_gemm<256, kResidue>(pa, pb, nmod, nmod, L.ldp, rows, cols, k, pl, nullptr, 0,
@@ -422,7 +436,7 @@ int ozaki2_multiply(int m, int k, int n, int nmod, const void* ws, size_t ws_byt
 
 // Rows [r0, r0 + rows) of C (dC its row 0) += CRT(R) * 2^(ea - ba + eb - bb).
 int ozaki2_reconstruct_rows(int m, int r0, int rows, int k, int n, double* dC, int64_t ldc, int nmod, const void* ws,
-                            size_t ws_bytes, cudaStream_t stream) {
+                            size_t ws_bytes, cudaStream_t stream, bool dependent) {
   Ozaki2Layout L;
   Ozaki2Views V;
   const int rc = ozaki2_views(m, k, n, nmod, ws, ws_bytes, L, V);
@@ -430,12 +444,13 @@ int ozaki2_reconstruct_rows(int m, int r0, int rows, int k, int n, double* dC, i
   if (r0 < 0 || rows <= 0 || r0 + rows > m) return PHPC_ERR_ARG;
   const ModTable T = make_table(nmod, k);
   if (T.crt.L.np != crt_digits(T.n)) return PHPC_ERR_UNSUPPORTED;  // the kernels' digit count per modulus count
+  cudaError_t e = cudaSuccess;
   with_crt_moduli(T.n, [&](auto nm) {
-    crt_kernel<decltype(nm)::value><<<dim3(rows, ceil_div(n, 128 * kCrtCols)), 128, 0, stream>>>(
-        V.R + (int64_t)r0 * L.ldr, L.ldr, (int64_t)m * L.ldr, rows, n, V.ea + r0, V.ba + r0, V.eb, V.bb, T,
-        dC + (int64_t)r0 * ldc, ldc);
+    e = launch_dependent(dependent, crt_kernel<decltype(nm)::value>, dim3(rows, ceil_div(n, 128 * kCrtCols)), 128, 0,
+                         stream, V.R + (int64_t)r0 * L.ldr, L.ldr, (int64_t)m * L.ldr, rows, n, V.ea + r0, V.ba + r0,
+                         V.eb, V.bb, T, dC + (int64_t)r0 * ldc, ldc);
   });
-  PHPC_CUDA_TRY(cudaGetLastError());
+  PHPC_CUDA_TRY(e);
   return PHPC_OK;
 }
 
@@ -458,11 +473,18 @@ int ozaki2_reconstruct(int m, int k, int n, double* dC, int64_t ldc, int nmod, c
   return ozaki2_reconstruct_rows(m, 0, m, k, n, dC, ldc, nmod, ws, ws_bytes, stream);
 }
 
+// In a short call each launch after the first comes up while the one before it
+// finishes (the GEMM's set-up of 208 KB of shared memory, barriers and TMEM
+// among it): N = 256 24.6 -> 20 us.
 int dgemm_ozaki2(int m, int k, int n, const double* dA, int64_t lda, const double* dB, int64_t ldb, double* dC,
                  int64_t ldc, int nmod, void* ws, size_t ws_bytes, cudaStream_t stream, int bn) {
-  int rc = ozaki2_prepare_on(m, k, n, dA, lda, dB, ldb, nmod, ws, ws_bytes, stream);
-  if (rc == PHPC_OK) rc = ozaki2_multiply(m, k, n, nmod, ws, ws_bytes, stream, bn);
-  if (rc == PHPC_OK) rc = ozaki2_reconstruct(m, k, n, dC, ldc, nmod, ws, ws_bytes, stream);
+  const DeviceInfo* dev = current_device();
+  if (!dev) return PHPC_ERR_CUDA;
+  bool joined = false;
+  const bool is_short = short_gemm(m, n, (int64_t)nmod * ceil_div(k, 64), dev->sm_count);
+  int rc = ozaki2_prepare_on(m, k, n, dA, lda, dB, ldb, nmod, ws, ws_bytes, stream, &joined);
+  if (rc == PHPC_OK) rc = ozaki2_multiply_block(m, 0, m, 0, n, k, n, nmod, ws, ws_bytes, stream, bn, !joined);
+  if (rc == PHPC_OK) rc = ozaki2_reconstruct_rows(m, 0, m, k, n, dC, ldc, nmod, ws, ws_bytes, stream, is_short);
   return rc;
 }
 

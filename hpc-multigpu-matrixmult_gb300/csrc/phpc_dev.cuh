@@ -32,6 +32,15 @@ __device__ __forceinline__ uint64_t globaltimer_ns() {
 
 __device__ __forceinline__ uint32_t elect_lane0() { return (threadIdx.x & 31) == 0; }
 
+// ------------------------------------------------ programmatic dependent launch
+// A kernel launched with launch_dependent (phpc_host.hpp) may start while the
+// kernel before it on the stream still runs: it touches no global memory
+// before pdl_wait, which returns when that kernel has completed (and with it,
+// since every kernel waits, all before it). pdl_trigger lets the next kernel
+// come up as soon as every CTA of this one has started.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---------------------------------------------------------------- status word
 __device__ __forceinline__ void record_error(int* status, int code) {
   if (status) atomicCAS(status, 0, code);

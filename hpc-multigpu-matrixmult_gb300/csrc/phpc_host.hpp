@@ -9,6 +9,7 @@
 #include <atomic>
 #include <cstdint>
 #include <cstdio>
+#include <utility>
 
 #include "phpc_gemm.h"
 
@@ -30,6 +31,40 @@ struct DeviceInfo {
   size_t smem_optin;
 };
 const DeviceInfo* current_device();
+
+inline int ceil_div(int64_t a, int64_t b) { return static_cast<int>((a + b - 1) / b); }
+
+// Launches a kernel; with `dependent` it may come up while the kernel before it
+// on the stream finishes (programmatic dependent launch: the kernel calls
+// pdl_wait before it touches global memory). Only for a kernel that directly
+// follows one of this library's own on the stream.
+template <class... P, class... A>
+cudaError_t launch_dependent(bool dependent, void (*kern)(P...), dim3 grid, dim3 block, size_t smem,
+                             cudaStream_t stream, A&&... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = dependent ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...);
+}
+
+// Whether a GEMM of `steps` K-steps a tile is short enough for dependent
+// launches around it: up to 80 K-steps an SM. A dependent launch takes the SMs
+// in the order they fall free instead of the regular one, and a long kernel
+// loses more by that (blocks that share data in L2 end up on different halves
+// of the GPU) than the set-up it hides: N = 1024 (44 K-steps an SM) 65.9 ->
+// 63.5 us, but 1537 x 1000 x 2311 (178) 161 -> 167-170, 4096 x 512 x 4096 330
+// -> 361, 3xBF16 at 32768 x 4096 x 8192 8.84 -> 9.12 ms with every launch
+// dependent.
+inline bool short_gemm(int m, int n, int64_t steps, int sms) {
+  return (int64_t)ceil_div(m, 128) * ceil_div(n, 256) * steps <= (int64_t)80 * sms;
+}
 
 // A value of 1 and up kept per device ordinal (a kernel attribute, an
 // occupancy): 0 until it is stored. Devices beyond the table are asked anew.
@@ -84,9 +119,9 @@ int ozaki2_multiply_rows(int m, int r0, int rows, int k, int n, int nmod, const 
 int ozaki2_prepare_b_cols(int m, int k, int n, int c0, int cols, const double* dB, int64_t ldb, int nmod, void* ws,
                           size_t ws_bytes, cudaStream_t stream);
 int ozaki2_multiply_block(int m, int r0, int rows, int c0, int cols, int k, int n, int nmod, const void* ws,
-                          size_t ws_bytes, cudaStream_t stream, int bn);
+                          size_t ws_bytes, cudaStream_t stream, int bn, bool dependent = false);
 int ozaki2_reconstruct_rows(int m, int r0, int rows, int k, int n, double* dC, int64_t ldc, int nmod, const void* ws,
-                            size_t ws_bytes, cudaStream_t stream);
+                            size_t ws_bytes, cudaStream_t stream, bool dependent = false);
 int ozaki2_reconstruct(int m, int k, int n, double* dC, int64_t ldc, int nmod, const void* ws, size_t ws_bytes,
                        cudaStream_t stream);
 int ozaki2_grids(int m, int k, int n, int nmod, const void* ws, size_t ws_bytes, int* ea, int* eb, int* ba, int* bb);
@@ -140,6 +175,5 @@ inline int64_t plane_ld(int k, bool padded) {
   return (k + to - 1) / to * to;
 }
 
-inline int ceil_div(int64_t a, int64_t b) { return static_cast<int>((a + b - 1) / b); }
 
 }  // namespace phpc

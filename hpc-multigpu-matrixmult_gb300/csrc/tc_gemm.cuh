@@ -331,6 +331,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     }
     fence_mbar_init();
   }
+  if (!GROUPED) pdl_trigger();
   if (warp == 1) {
     if (CLUSTER == 1)
       tmem_alloc(tmem_slot, Cfg::kTmemCols);
@@ -342,6 +343,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   if (CLUSTER > 1) cluster_sync();  // peer barriers initialised and TMEM allocated in both CTAs
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  if (!GROUPED) pdl_wait();  // everything before reads or writes no global memory
   bool pair_ok = true;
   if (CLUSTER > 1) {
     // The pair's MMAs address the same TMEM columns in both CTAs; refuse to run
@@ -917,6 +919,7 @@ inline bool encode_residue_planes(CUtensorMap* map, const uint16_t* R, int m, in
 struct TcGemmOpts {
   int64_t a_plane_rows = 0;            // rows between consecutive A planes (0: m, the planes are m rows high)
   int64_t b_plane_rows = 0;            // rows between consecutive B planes (0: n)
+  bool dependent = false;              // the planes' split directly precedes on the stream (launch_dependent)
   int cfg_m = 0, cfg_n = 0, cfg_k = 0;  // shape whose tuning entry sets cluster and raster (0: this GEMM's)
 };
 
