@@ -2,10 +2,10 @@
 //
 // Replaces the reference's SIMT kernel (src/phpc_gemm.cu:6-57, shared-memory
 // tiles of tile_width^2 doubles, one DFMA per shared load pair) with:
-//  - a persistent grid that walks the output tiles of the logical SUMMA block
-//    grid (grid_width x grid_height blocks of C, src/phpc_summa.c:36-44),
-//    block by block, so the CTAs working at one time share A row panels and
-//    B column panels in L2;
+//  - one CTA per output tile, numbered through the logical SUMMA block grid
+//    (grid_width x grid_height blocks of C, src/phpc_summa.c:36-44) block by
+//    block, so the CTAs working at one time share A row panels and B column
+//    panels in L2;
 //  - a producer warp that streams the k-panels of A and B into a shared-memory
 //    ring of 2-6 stages (4 unless PHPC_DMMA_STAGES or the tuning table's
 //    "plain" entry says otherwise) with TMA (the on-device form of the reference's
@@ -58,7 +58,7 @@ __device__ __forceinline__ void tile_coords(const SummaGrid& g, int t, int& rm, 
 // SM's four quarters has its own FP64 pipe (half an FMA a clock), so both
 // tiles give every quarter a warp (FP64 tensor-core warps are at least
 // 16 x 8). Larger tiles buy nothing, since the pipe, not shared memory or L2,
-// is the limit: 64 x 64 tiles took 14.4 ms at N = 2048 against 14.05 for
+// is the limit: 64 x 64 tiles took 14.4 ms at N = 2048 against 13.8 for
 // 16 x 16, 128 x 128 tiles 895 ms at N = 8192 against 883 for 32 x 32, and a
 // call that leaves SMs idle at 64 x 64 is up to 8x slower (250 x 514 x 302:
 // 566 us against 73.6).
@@ -101,7 +101,8 @@ __global__ void __launch_bounds__(DmmaCfg<BT, DFMA>::kThreads)
   uint64_t* empty = full + S;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int ntiles = grid.tm * grid.tn;
+  int rm, rn;
+  tile_coords(grid, blockIdx.x, rm, rn);
   const int ksteps = (K + kBK - 1) / kBK;
   const int kp_steps = max(1, kpanel / kBK);  // BK steps per SUMMA k-panel
 
@@ -123,21 +124,17 @@ __global__ void __launch_bounds__(DmmaCfg<BT, DFMA>::kThreads)
       uint32_t phase = 0;
       int issued = 0;
       bool ok = true;
-      for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
-        int rm, rn;
-        tile_coords(grid, t, rm, rn);
-        // SUMMA k-panels, each streamed as kp_steps TMA stages.
-        for (int p0 = 0; p0 < ksteps && ok; p0 += kp_steps) {
-          const int p1 = min(ksteps, p0 + kp_steps);
-          for (int ks = p0; ks < p1; ++ks) {
-            if (!wait_parity(&empty[stage], phase ^ 1, status, 1)) { ok = false; break; }
-            mbar_arrive_expect_tx(&full[stage], Cfg::kStageBytes);
-            uint8_t* sa = smem + stage * Cfg::kStageBytes;
-            tma_load_2d(sa, &tmA, ks * kBK, rm * BM, &full[stage]);
-            tma_load_2d(sa + Cfg::kStageA, &tmB, rn * BN, ks * kBK, &full[stage]);
-            ++issued;
-            if (++stage == S) { stage = 0; phase ^= 1; }
-          }
+      // SUMMA k-panels, each streamed as kp_steps TMA stages.
+      for (int p0 = 0; p0 < ksteps && ok; p0 += kp_steps) {
+        const int p1 = min(ksteps, p0 + kp_steps);
+        for (int ks = p0; ks < p1; ++ks) {
+          if (!wait_parity(&empty[stage], phase ^ 1, status, 1)) { ok = false; break; }
+          mbar_arrive_expect_tx(&full[stage], Cfg::kStageBytes);
+          uint8_t* sa = smem + stage * Cfg::kStageBytes;
+          tma_load_2d(sa, &tmA, ks * kBK, rm * BM, &full[stage]);
+          tma_load_2d(sa + Cfg::kStageA, &tmB, rn * BN, ks * kBK, &full[stage]);
+          ++issued;
+          if (++stage == S) { stage = 0; phase ^= 1; }
         }
       }
       if (!ok) {
@@ -159,78 +156,74 @@ __global__ void __launch_bounds__(DmmaCfg<BT, DFMA>::kThreads)
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;
-    for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
-      int rm, rn;
-      tile_coords(grid, t, rm, rn);
-      double acc[NR][NJ][2];
+    double acc[NR][NJ][2];
 #pragma unroll
-      for (int r = 0; r < NR; ++r)
+    for (int r = 0; r < NR; ++r)
 #pragma unroll
-        for (int j = 0; j < NJ; ++j) acc[r][j][0] = acc[r][j][1] = 0.0;
+      for (int j = 0; j < NJ; ++j) acc[r][j][0] = acc[r][j][1] = 0.0;
 
-      for (int ks = 0; ks < ksteps; ++ks) {
-        // all lanes must agree before the warp-collective mma.sync below
-        ok = __all_sync(0xffffffffu, wait_parity(&full[stage], phase, status, 2));
-        if (!ok) break;
-        const double* sA = reinterpret_cast<const double*>(smem + stage * Cfg::kStageBytes);  // [BM][16]
-        const double* sB = reinterpret_cast<const double*>(smem + stage * Cfg::kStageBytes + Cfg::kStageA);  // [16][BN]
-        if (DFMA) {
+    for (int ks = 0; ks < ksteps; ++ks) {
+      // all lanes must agree before the warp-collective mma.sync below
+      ok = __all_sync(0xffffffffu, wait_parity(&full[stage], phase, status, 2));
+      if (!ok) break;
+      const double* sA = reinterpret_cast<const double*>(smem + stage * Cfg::kStageBytes);  // [BM][16]
+      const double* sB = reinterpret_cast<const double*>(smem + stage * Cfg::kStageBytes + Cfg::kStageA);  // [16][BN]
+      if (DFMA) {
 #pragma unroll 2
-          for (int c = 0; c < kBK / 2; ++c) {
-            double2 a[NR];
+        for (int c = 0; c < kBK / 2; ++c) {
+          double2 a[NR];
+#pragma unroll
+          for (int r = 0; r < NR; ++r)
+            a[r] = *reinterpret_cast<const double2*>(a_chunk(sA, wm * WM + 8 * r + g, c));
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            double2 b[NJ];
+#pragma unroll
+            for (int j = 0; j < NJ; ++j)
+              b[j] = *reinterpret_cast<const double2*>(&sB[(2 * c + h) * BN + wn * WN + j * 8 + 2 * tig]);
 #pragma unroll
             for (int r = 0; r < NR; ++r)
-              a[r] = *reinterpret_cast<const double2*>(a_chunk(sA, wm * WM + 8 * r + g, c));
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              double2 b[NJ];
-#pragma unroll
-              for (int j = 0; j < NJ; ++j)
-                b[j] = *reinterpret_cast<const double2*>(&sB[(2 * c + h) * BN + wn * WN + j * 8 + 2 * tig]);
-#pragma unroll
-              for (int r = 0; r < NR; ++r)
-#pragma unroll
-                for (int j = 0; j < NJ; ++j) {
-                  acc[r][j][0] = fma(h ? a[r].y : a[r].x, b[j].x, acc[r][j][0]);
-                  acc[r][j][1] = fma(h ? a[r].y : a[r].x, b[j].y, acc[r][j][1]);
-                }
-            }
-          }
-        } else {
-#pragma unroll
-          for (int kk = 0; kk < kBK; kk += 4) {
-            double a[NR], b[NJ];
-#pragma unroll
-            for (int r = 0; r < NR; ++r) a[r] = a_chunk(sA, wm * WM + 8 * r + g, (kk + tig) >> 1)[tig & 1];
-#pragma unroll
-            for (int j = 0; j < NJ; ++j) b[j] = sB[(kk + tig) * BN + wn * WN + j * 8 + g];
-#pragma unroll
-            for (int r = 0; r + 1 < NR; r += 2)
-#pragma unroll
-              for (int j = 0; j < NJ; ++j)
-                asm volatile(
-                    "mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
-                    : "+d"(acc[r][j][0]), "+d"(acc[r][j][1]), "+d"(acc[r + 1][j][0]), "+d"(acc[r + 1][j][1])
-                    : "d"(a[r]), "d"(a[r + 1]), "d"(b[j]));
+              for (int j = 0; j < NJ; ++j) {
+                acc[r][j][0] = fma(h ? a[r].y : a[r].x, b[j].x, acc[r][j][0]);
+                acc[r][j][1] = fma(h ? a[r].y : a[r].x, b[j].y, acc[r][j][1]);
+              }
           }
         }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&empty[stage]);
-        if (++stage == S) { stage = 0; phase ^= 1; }
+      } else {
+#pragma unroll
+        for (int kk = 0; kk < kBK; kk += 4) {
+          double a[NR], b[NJ];
+#pragma unroll
+          for (int r = 0; r < NR; ++r) a[r] = a_chunk(sA, wm * WM + 8 * r + g, (kk + tig) >> 1)[tig & 1];
+#pragma unroll
+          for (int j = 0; j < NJ; ++j) b[j] = sB[(kk + tig) * BN + wn * WN + j * 8 + g];
+#pragma unroll
+          for (int r = 0; r + 1 < NR; r += 2)
+#pragma unroll
+            for (int j = 0; j < NJ; ++j)
+              asm volatile(
+                  "mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
+                  : "+d"(acc[r][j][0]), "+d"(acc[r][j][1]), "+d"(acc[r + 1][j][0]), "+d"(acc[r + 1][j][1])
+                  : "d"(a[r]), "d"(a[r + 1]), "d"(b[j]));
+        }
       }
-      if (!ok) break;
-      // Epilogue: C += tile.
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&empty[stage]);
+      if (++stage == S) { stage = 0; phase ^= 1; }
+    }
+    if (!ok) return;
+    // Epilogue: C += tile.
 #pragma unroll
-      for (int r = 0; r < NR; ++r) {
-        const int64_t row = (int64_t)rm * BM + wm * WM + 8 * r + g;
-        if (row >= M) continue;
-        double* crow = C + row * ldc;
+    for (int r = 0; r < NR; ++r) {
+      const int64_t row = (int64_t)rm * BM + wm * WM + 8 * r + g;
+      if (row >= M) continue;
+      double* crow = C + row * ldc;
 #pragma unroll
-        for (int j = 0; j < NJ; ++j) {
-          const int col = rn * BN + wn * WN + j * 8 + 2 * tig;
-          if (col < N) crow[col] += acc[r][j][0];
-          if (col + 1 < N) crow[col + 1] += acc[r][j][1];
-        }
+      for (int j = 0; j < NJ; ++j) {
+        const int col = rn * BN + wn * WN + j * 8 + 2 * tig;
+        if (col < N) crow[col] += acc[r][j][0];
+        if (col + 1 < N) crow[col + 1] += acc[r][j][1];
       }
     }
   }
@@ -263,17 +256,16 @@ int launch_dmma(int m, int k, int n, const double* dA, int64_t lda, const double
   const int stages = default_plain_stages(m, k, n);
   if (stages < 2 || stages > kMaxStages) return PHPC_ERR_ARG;
   const size_t smem = Cfg::smem(stages);
-  static PerDevice blocks_per_sm[kMaxStages + 1];
-  int per_sm = blocks_per_sm[stages].get(dev->ordinal);
-  if (per_sm == 0) {
+  static PerDevice ready;
+  if (!ready.get(dev->ordinal)) {
     PHPC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::smem(kMaxStages)));
-    PHPC_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, Cfg::kThreads, smem));
-    per_sm = std::max(1, per_sm);
-    blocks_per_sm[stages].set(dev->ordinal, per_sm);
+    ready.set(dev->ordinal, 1);
   }
-  const int nblocks = std::min(ntiles, dev->sm_count * per_sm);
-  kern<<<nblocks, Cfg::kThreads, smem, stream>>>(tmA, tmB, dC, ldc, m, n, k, kpanel, g, stages,
-                                                                             device_status_ptr());
+  // One CTA per tile: the hardware gives an SM its next tile when one is done.
+  // A persistent grid with tiles c, c + grid, ... left some SMs 8 % more work
+  // (N = 1024 1806 us against 1745, 2048 14.05 ms against 13.84), and a CTA's
+  // set-up is hidden by the seven others on its SM.
+  kern<<<ntiles, Cfg::kThreads, smem, stream>>>(tmA, tmB, dC, ldc, m, n, k, kpanel, g, stages, device_status_ptr());
   PHPC_CUDA_TRY(cudaGetLastError());
   return PHPC_OK;
 }
@@ -290,13 +282,13 @@ bool fp64_pipe_is_dfma() {
 // Tile side: a call takes as long as the SM with the most outputs (padding
 // included), ceil(tiles / SMs) x BT^2, so the smaller tile is never behind by
 // load (N = 1024 in 64 x 64 tiles: 2104 us, 2 tiles on some SMs, 1 on others;
-// in 16 x 16: 1813). From 128 tiles of 32 x 32 an SM that difference is under
-// 1 % and the larger tile's fewer loads count for more (N = 4096, 108 tiles an
-// SM: 16 111.0 ms, 32 111.6; N = 8192: 887 and 883). PHPC_DMMA_TILE = 16 forces
-// the one, any other number the other.
+// in 16 x 16: 1745). From 100 tiles of 32 x 32 an SM that difference is under
+// 1 % and the larger tile's fewer loads count for more (N = 3000, 58 tiles an
+// SM, K = 500: 16 7.49 ms, 32 7.55; N = 4096, 108 an SM: 110.4 and 110.15).
+// PHPC_DMMA_TILE = 16 forces the one, any other number the other.
 int plain_tile(int m, int n, int sms) {
   if (const char* force = getenv("PHPC_DMMA_TILE")) return atoi(force) == 16 ? 16 : 32;
-  return (int64_t)ceil_div(m, 32) * ceil_div(n, 32) >= (int64_t)128 * sms ? 32 : 16;
+  return (int64_t)ceil_div(m, 32) * ceil_div(n, 32) >= (int64_t)100 * sms ? 32 : 16;
 }
 
 int dgemm_dmma(int m, int k, int n, const double* dA, int64_t lda, const double* dB, int64_t ldb, double* dC,
