@@ -94,6 +94,9 @@ __device__ __forceinline__ bool wait_parity(uint64_t* bar, uint32_t parity, int*
 }
 
 // ----------------------------------------------------------------------- TMA
+// Brings the line at p into L2 (a hint; nothing waits for it).
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 __device__ __forceinline__ void tma_prefetch_desc(const void* tmap) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(tmap)) : "memory");
 }

@@ -601,6 +601,20 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         const int chunk = MODE == kOzaki ? kTcChunkSteps : MODE == kResidue ? kTcResidueChunkSteps : KSPLIT ? kTcKsplitChunkSteps : kTcF32ChunkSteps;
         const int nchunks = (total + chunk - 1) / chunk;
         for (int c = 0; c < nchunks && ok; ++c) {
+          if (MODE == kF32 && !KSPLIT && c == max(nchunks - 2, 0)) {
+            // The warp's part of C into L2 while the last two chunks are computed:
+            // every CTA reaches its epilogue at about the same time, and the
+            // reads' DRAM latency was half of what the MMAs then wait for
+            // (epilogue below). A tile further ahead was slower (165 us against
+            // 155 at 5505 x 333 x 5671).
+            const float* Cf = static_cast<const float*>(job.C) + (row0 + lane) * job.ldc + col0;
+            if (row0 + lane < job.M) {
+#pragma unroll
+              for (int e = 0; e < HALF; e += 32)
+                if (col0 + e < job.N) prefetch_l2(Cf + e);
+              if (col0 + HALF <= job.N) prefetch_l2(Cf + HALF - 1);
+            }
+          }
           // all lanes must agree before the warp-collective tcgen05.ld below
           ok = __all_sync(0xffffffffu, wait_parity(&tfull[buf], tphase[buf], status, 14));
           if (!ok) break;
@@ -757,7 +771,11 @@ __global__ void __launch_bounds__(kTcThreads, 1)
           }
           // Write the warp's 32 rows x HALF columns out, 32 columns at a time,
           // transposed through shared memory so that a warp touches one
-          // contiguous 32-element run of a row per access.
+          // contiguous 32-element run of a row per access. kF32: of short K this
+          // sets the pace (the MMAs run at most two chunks ahead of it): with the
+          // lines in L2 already and the addresses stepped by ldc 8192 x 128 x
+          // 8192 takes 169 us instead of 253, 5505 x 333 x 5671 149 instead of
+          // 185, 4096^3 620 instead of 638. 32 rows in flight spill (155, 625).
           const int gexp = MODE == kOzaki ? 2 - 8 * (int)pairs.g[gstart] : 0;
           constexpr int kBatch = 16;  // rows whose C loads are in flight together
 #pragma unroll
@@ -791,18 +809,15 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                         fold_add(cv[u], (int32_t)tr[(r0 + u) * 33 + lane], row_e + col_e + gexp);
                 }
               } else {
-                float* Cf = static_cast<float*>(job.C);
+                float* Cf = static_cast<float*>(job.C) + (row0 + r0) * job.ldc + col;
+                const int rows = col_ok ? static_cast<int>(min((int64_t)kBatch, job.M - row0 - r0)) : 0;
                 float cv[kBatch];
+                const float* src = Cf;
 #pragma unroll
-                for (int u = 0; u < kBatch; ++u) {
-                  const int64_t grow = row0 + r0 + u;
-                  cv[u] = (grow < job.M && col_ok) ? Cf[grow * job.ldc + col] : 0.f;
-                }
+                for (int u = 0; u < kBatch; ++u, src += job.ldc) cv[u] = u < rows ? *src : 0.f;
 #pragma unroll
-                for (int u = 0; u < kBatch; ++u) {
-                  const int64_t grow = row0 + r0 + u;
-                  if (grow < job.M && col_ok) Cf[grow * job.ldc + col] = cv[u] + __uint_as_float(tr[(r0 + u) * 33 + lane]);
-                }
+                for (int u = 0; u < kBatch; ++u, Cf += job.ldc)
+                  if (u < rows) *Cf = cv[u] + __uint_as_float(tr[(r0 + u) * 33 + lane]);
               }
             }
             __syncwarp();
