@@ -66,6 +66,7 @@ struct PrepCols {
 };
 
 constexpr int kPrepThreads = 256;
+constexpr int kOneStreamK = 2560;  // ozaki2_prepare_on
 constexpr int kScanRowsPerBlock = kPrepThreads / 32;  // one warp per row
 
 // Row blocks: one warp per row of A: ea[i] = max_k e(A[i][k]) and the row's
@@ -360,9 +361,12 @@ int ozaki2_prepare2(int m, int k, int n, const double* dA, int64_t lda, const do
 }
 
 // The same on one caller stream. Small operands (below 32 MB together, and K
-// <= 1024: no merge kernel between scan and split) share the two launches:
-// the fork and join cost more than the overlap gives (N = 256 53 -> 42 us,
-// 1537 x 1000 x 2311 169.7 -> 168.5, but 4096 x 512 x 4096 360 -> 364). Above,
+// <= 2560) share the two or three launches: the fork and join cost more than
+// the overlap gives (prepare alone, two streams / one: N = 256 13.5, 8.7 us;
+// 664 x 1420 x 668 26.8, 22.9; 1537 x 1000 x 2311 40.3, 37.3; but 4096 x 1024 x
+// 4096 72.1, 74.2). With longer rows a warp's scan of one row, which B's work
+// on the other stream hides, takes as long as they do (569 x 3453 x 178 31.3,
+// 33.1; 387 x 5556 x 580 53.7, 59.8; 256 x 8192 x 256 47.6, 55.8). Above,
 // B's scans and split run on this thread's side stream beside A's (both are
 // memory-bound; run together, one's ramp-up and tail overlap the other's), and
 // the caller's stream waits for them.
@@ -371,7 +375,7 @@ int ozaki2_prepare2(int m, int k, int n, const double* dA, int64_t lda, const do
 int ozaki2_prepare_on(int m, int k, int n, const double* dA, int64_t lda, const double* dB, int64_t ldb, int nmod,
                       void* ws, size_t ws_bytes, cudaStream_t stream, bool* joined = nullptr) {
   if (joined) *joined = false;
-  if (ceil_div(k, kNormChunk) <= kMergeInSplit && ((int64_t)m + n) * k < (4 << 20)) {
+  if (k <= kOneStreamK && ((int64_t)m + n) * k < (4 << 20)) {
     Ozaki2Layout L;
     Ozaki2Views V;
     const int rc = ozaki2_views(m, k, n, nmod, ws, ws_bytes, L, V);
