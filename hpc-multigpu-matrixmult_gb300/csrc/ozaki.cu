@@ -121,12 +121,12 @@ constexpr int kMaxKsplit = 8;
 
 // Clusters of `split` K-splitting CTAs that run at one time (the clusters of
 // one GPC share its SMs, so this is below SMs / split); asked once a device.
-template <int BN>
+template <int BN, int MODE>
 int ksplit_clusters(int split, const DeviceInfo* dev) {
   static PerDevice cached[kMaxKsplit + 1];  // clusters + 1
   int n = cached[split].get(dev->ordinal);
   if (n > 0) return n - 1;
-  constexpr auto kern = tc_slice_gemm_kernel<BN, kF32, false, 1, true>;
+  constexpr auto kern = tc_slice_gemm_kernel<BN, MODE, false, 1, true>;
   cudaLaunchAttribute attr[1];
   const cudaLaunchConfig_t cfg = ksplit_config<BN>(split, attr);
   if (tc_ready<kern>(dev, TcCfg<BN>::kSmem) != PHPC_OK ||
@@ -156,7 +156,26 @@ int f32_ksplit(int m, int n, int steps, const DeviceInfo* dev) {
   if (env && atoi(env) >= 1 && atoi(env) <= kMaxKsplit) return std::min(atoi(env), steps);
   const int64_t tiles = (int64_t)ceil_div(m, kTcBM) * ceil_div(n, 256);
   for (int s = kMaxKsplit; s > 1; --s)
-    if (tiles * s <= dev->sm_count && steps >= 48 && steps / s >= 4 && tiles <= ksplit_clusters<BN>(s, dev)) return s;
+    if (tiles * s <= dev->sm_count && steps >= 48 && steps / s >= 4 && tiles <= ksplit_clusters<BN, kF32>(s, dev)) return s;
+  return 1;
+}
+
+// The same for a residue GEMM whose (tile, modulus) units leave SMs idle. A
+// K-step takes 0.33 us whatever the tile width (48 KB, or 32, at an SM's share
+// of the L2 rate), and the shares' exchange through shared memory 4-6 us, so it
+// pays from 40 steps (K > 2496). GEMM alone, unsplit / split: 128 x 8192 x 128
+// 45.3 us, 20.9 with 8; 256 x 8192 x 256 53.8, 29.4 with 4; 336 x 4001 x 72
+// 26.8, 20.6 with 3; 235 x 3167 x 169 22.7, 18.6 with 3; 569 x 3453 x 178 24.7,
+// 22.7 with 2; but 128 x 2048 x 128 16.5, 16.9 with 8, and 640 x 1500 x 256
+// 14.8, 18.5 with 2. The residues are exact, so the bits do not depend on it.
+// PHPC_RESIDUE_KSPLIT = 1..8 forces it.
+template <int BN>
+int residue_ksplit(int64_t units, int steps, const DeviceInfo* dev) {
+  const char* env = getenv("PHPC_RESIDUE_KSPLIT");
+  if (env && atoi(env) >= 1 && atoi(env) <= kMaxKsplit) return std::min(atoi(env), steps);
+  for (int s = kMaxKsplit; s > 1; --s)
+    if (units * s <= dev->sm_count && steps >= 40 && units <= ksplit_clusters<BN, kResidue>(s, dev))
+      return s;
   return 1;
 }
 
@@ -224,15 +243,18 @@ int launch_tc_slice_gemm(const void* planesA, const void* planesB, int nplanesA,
   const int64_t units =
       (cluster == 1 ? (int64_t)a.tm * a.tn : (int64_t)((a.tm + 1) / 2) * a.tn) * (a.split_pairs ? pairs.n : 1);
   const bool dependent = opt.dependent && short_gemm(m, n, pairs.n * ceil_div(k, kTcBK), dev->sm_count);
-  if constexpr (MODE == kF32) {
-    a.ksplit = f32_ksplit<BN>(m, n, pairs.n * ceil_div(k, kTcBK), dev);
+  if constexpr (MODE == kF32 || MODE == kResidue) {
+    if (MODE == kF32)
+      a.ksplit = f32_ksplit<BN>(m, n, pairs.n * ceil_div(k, kTcBK), dev);
+    else
+      a.ksplit = cluster == 1 && a.split_pairs ? residue_ksplit<BN>(units, ceil_div(k, kTcBK), dev) : 1;
     if (a.ksplit > 1) {
       constexpr auto kern = tc_slice_gemm_kernel<BN, MODE, false, 1, true>;
       if (const int rc = tc_ready<kern>(dev, Cfg::kSmem); rc != PHPC_OK) return rc;
       cudaLaunchAttribute attr[2];
       cudaLaunchConfig_t cfg = ksplit_config<BN>(a.ksplit, attr);
       if (dependent) dependent_attr(attr, cfg);
-      cfg.gridDim = dim3(static_cast<unsigned>(a.tm * a.tn * a.ksplit), 1, 1);
+      cfg.gridDim = dim3(static_cast<unsigned>(units * a.ksplit), 1, 1);
       cfg.stream = stream;
       PHPC_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, tmA, tmB, tmR, pairs, a, TcGroupTable{}));
       return PHPC_OK;

@@ -108,7 +108,7 @@ struct TcArgs {
   int64_t rplane;             // kResidue: plane stride in elements
   int split_pairs;            // kResidue: a work unit is one (tile, modulus), moduli outer
   int stages;                 // K-stages of the ring in use, 2 .. TcCfg::kStages (other values: kStages)
-  int ksplit;                 // KSPLIT: CTAs (one cluster) per tile
+  int ksplit;                 // KSPLIT: CTAs (one cluster) per unit
   int k_serpentine;           // kResidue: every other round of units walks K from the end (see the producer)
 };
 
@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                          const __grid_constant__ CUtensorMap tmR, const __grid_constant__ PairList pairs, const __grid_constant__ TcArgs args,
                          const __grid_constant__ TcGroupTable gt) {
   static_assert(CLUSTER == 1 || (CLUSTER == 2 && !GROUPED), "the CTA pair computes tiles of one problem");
-  static_assert(!KSPLIT || (MODE == kF32 && CLUSTER == 1 && !GROUPED), "K is split in the FP32 GEMM only");
+  static_assert(!KSPLIT || (MODE != kOzaki && CLUSTER == 1 && !GROUPED), "K is split in the FP32 and residue GEMMs only");
   using Cfg = TcCfg<BN, CLUSTER>;
   // The shared-memory layout is that of the deepest ring; the ring in use has
   // S stages (the tuning table's pipeline depth).
@@ -308,9 +308,9 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   const bool leader = crank == 0;
   const int unit0 = CLUSTER > 1 || KSPLIT ? static_cast<int>(cluster_id_x()) : static_cast<int>(blockIdx.x);
   const int ustride = CLUSTER > 1 || KSPLIT ? static_cast<int>(nclusters_x()) : static_cast<int>(gridDim.x);
-  // KSPLIT (one tile per cluster): this CTA's share [ks0, ks1) of the tile's steps
+  // KSPLIT (one unit per cluster): this CTA's share [ks0, ks1) of the unit's steps
   const int krank = KSPLIT ? static_cast<int>(cluster_ctarank()) : 0;
-  const int ksteps = KSPLIT ? pairs.n * ((args.K + kTcBK - 1) / kTcBK) : 0;
+  const int ksteps = KSPLIT ? (MODE == kResidue ? 1 : pairs.n) * ((args.K + kTcBK - 1) / kTcBK) : 0;
   const int ks0 = KSPLIT ? ksteps * krank / args.ksplit : 0, ks1 = KSPLIT ? ksteps * (krank + 1) / args.ksplit : 0;
   const int ntiles = GROUPED ? gt.ntiles : (CLUSTER > 1 ? (args.tm + 1) / 2 : args.tm) * args.tn;
   int* status = args.status;
@@ -419,8 +419,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         const bool rev = serp && (round & 1);
         for (int pi = p0; pi < p1 && ok; ++pi) {
           const int pa = pairs.a[pi], pb = pairs.b[pi];
-          const int kb0 = KSPLIT ? min(max(ks0 - pi * job.nk, 0), job.nk) : 0;
-          const int kb1 = KSPLIT ? min(max(ks1 - pi * job.nk, 0), job.nk) : job.nk;
+          const int kb0 = KSPLIT ? min(max(ks0 - (pi - p0) * job.nk, 0), job.nk) : 0;
+          const int kb1 = KSPLIT ? min(max(ks1 - (pi - p0) * job.nk, 0), job.nk) : job.nk;
           for (int kb = kb0; kb < kb1; ++kb) {
             if (!wait_parity(&empty[stage], phase ^ 1, status, 11)) { ok = false; break; }
             uint8_t* sa = smem + stage * Cfg::kStageBytes;
@@ -495,7 +495,10 @@ __global__ void __launch_bounds__(kTcThreads, 1)
           else
             gend = p1;
           const int total = KSPLIT ? ks1 - ks0 : (gend - gstart) * nk;
-          const int chunk = MODE == kOzaki ? kTcChunkSteps : MODE == kResidue ? kTcResidueChunkSteps : KSPLIT ? kTcKsplitChunkSteps : kTcF32ChunkSteps;
+          const int chunk = MODE == kOzaki     ? kTcChunkSteps
+                              : MODE == kResidue ? kTcResidueChunkSteps
+                              : KSPLIT           ? kTcKsplitChunkSteps
+                                                 : kTcF32ChunkSteps;
           for (int done = 0; done < total && ok; done += chunk) {
             const int len = min(chunk, total - done);
             if (!wait_parity(&tempty[buf], tphase[buf] ^ 1, status, 12)) { ok = false; break; }
@@ -561,6 +564,15 @@ __global__ void __launch_bounds__(kTcThreads, 1)
 #pragma unroll
     for (int j = 0; j < HALF; ++j) acc[j] = 0;
 
+    const auto put_share = [&]() {  // KSPLIT: this warp's sums into shared memory, for the cluster
+      // every MMA of this CTA has read its operands: the ring is free
+      const int r = quad * 32 + lane;
+#pragma unroll
+      for (int c = 0; c < HALF / 4; ++c)
+        *reinterpret_cast<int4*>(smem + ksplit_chunk<BN>(r, half * (HALF / 4) + c)) =
+            make_int4(acc[4 * c], acc[4 * c + 1], acc[4 * c + 2], acc[4 * c + 3]);
+    };
+
     uint32_t qphase = 0;
     for (int i = 0; ok; ++i) {
       int u;
@@ -598,7 +610,10 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         else
           gend = p1;
         const int total = KSPLIT ? ks1 - ks0 : (gend - gstart) * job.nk;
-        const int chunk = MODE == kOzaki ? kTcChunkSteps : MODE == kResidue ? kTcResidueChunkSteps : KSPLIT ? kTcKsplitChunkSteps : kTcF32ChunkSteps;
+        const int chunk = MODE == kOzaki     ? kTcChunkSteps
+                          : MODE == kResidue ? kTcResidueChunkSteps
+                          : KSPLIT           ? kTcKsplitChunkSteps
+                                             : kTcF32ChunkSteps;
         const int nchunks = (total + chunk - 1) / chunk;
         for (int c = 0; c < nchunks && ok; ++c) {
           if (MODE == kF32 && !KSPLIT && c == max(nchunks - 2, 0)) {
@@ -687,7 +702,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
           if (!fold) continue;
           if (MODE == kResidue) {
             const float mf = static_cast<float>(pairs.mod[gstart]), invm = pairs.invm[gstart];
-            if (!group_end) {  // keep the partial residue; more chunks of this modulus follow
+            if (!group_end || KSPLIT) {  // keep the partial residue; more chunks or shares of this modulus follow
 #pragma unroll
               for (int u = 0; u < HALF; u += 2) {
                 const float2 red =
@@ -695,6 +710,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                 acc[u] = __float_as_int(red.x);
                 acc[u + 1] = __float_as_int(red.y);
               }
+              if (KSPLIT && group_end) put_share();
               continue;
             }
             // One 16-bit value per element, 64 columns at a time: each lane
@@ -761,12 +777,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             continue;
           }
           if (KSPLIT) {
-            // every MMA of this CTA has read its operands: the ring is free
-            const int r = quad * 32 + lane;
-#pragma unroll
-            for (int c = 0; c < HALF / 4; ++c)
-              *reinterpret_cast<int4*>(smem + ksplit_chunk<BN>(r, half * (HALF / 4) + c)) =
-                  make_int4(acc[4 * c], acc[4 * c + 1], acc[4 * c + 2], acc[4 * c + 3]);
+            put_share();
             continue;
           }
           // Write the warp's 32 rows x HALF columns out, 32 columns at a time,
@@ -828,11 +839,13 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         gstart = gend;
       }
     }
-    if (MODE == kResidue && lane == 0) bulk_wait_all();  // the stores have left shared memory
+    if (MODE == kResidue && !KSPLIT && lane == 0) bulk_wait_all();  // the stores have left shared memory
     if (KSPLIT) {
       cluster_sync();  // every CTA's sums are in its shared memory
+      int t, p0;
+      tc_unit(unit0, ntiles, split, t, p0);
       TcJob job;
-      tc_job<GROUPED, CLUSTER>(unit0, args, &tmA, &tmB, &tmR, gt, crank, job);
+      tc_job<GROUPED, CLUSTER>(t, args, &tmA, &tmB, &tmR, gt, crank, job);
       const uint32_t base = smem_u32(smem);
       // this CTA's rows, four 16-byte chunks a thread at a time, four CTAs' sums
       // of each in flight, their C values on the way meanwhile
@@ -848,7 +861,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
           const int64_t row = (int64_t)job.rm * kTcBM + r;
 #pragma unroll
           for (int e = 0; e < 4; ++e)
-            cv[u][e] = r < r1 && row < job.M && col + e < job.N ? Cf[row * job.ldc + col + e] : 0.f;
+            cv[u][e] = MODE == kF32 && r < r1 && row < job.M && col + e < job.N ? Cf[row * job.ldc + col + e] : 0.f;
         }
         for (int q0 = 0; q0 < args.ksplit; q0 += 4) {
           float4 v[4][kBatch];
@@ -875,6 +888,23 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         for (int u = 0; u < kBatch; ++u) {
           const int i = i0 + u * kTcEpiWarps * 32, r = r0 + i / kChunks, col = job.rn * BN + 4 * (i % kChunks);
           const int64_t row = (int64_t)job.rm * kTcBM + r;
+          if (MODE == kResidue) {
+            // the shares' residues (at most 0.51 m each) add up exactly
+            const float mf = static_cast<float>(pairs.mod[p0]), invm = pairs.invm[p0];
+            const uint2 t4 = make_uint2(crt_t_pair(sum[u].x, sum[u].y, mf, invm),
+                                        crt_t_pair(sum[u].z, sum[u].w, mf, invm));
+            uint16_t* dst = job.R + static_cast<int64_t>(pairs.g[p0]) * job.rplane + row * job.ldr + col;
+            if (r >= r1 || row >= job.M) continue;
+            if (col + 4 <= job.N) {
+              *reinterpret_cast<uint2*>(dst) = t4;
+            } else {
+              const uint32_t src[2] = {t4.x, t4.y};
+#pragma unroll
+              for (int e = 0; e < 4; ++e)
+                if (col + e < job.N) dst[e] = static_cast<uint16_t>(src[e >> 1] >> (16 * (e & 1)));
+            }
+            continue;
+          }
           const float s4[4] = {sum[u].x, sum[u].y, sum[u].z, sum[u].w};
 #pragma unroll
           for (int e = 0; e < 4; ++e)
