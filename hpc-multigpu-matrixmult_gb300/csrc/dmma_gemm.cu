@@ -10,7 +10,7 @@
 //    ring of 2-6 stages (4 unless PHPC_DMMA_STAGES or the tuning table's
 //    "plain" entry says otherwise) with TMA (the on-device form of the reference's
 //    per-panel row/column broadcasts, src/phpc_summa.c:63-89);
-//  - consumer warps computing 8 x 8 to 16 x 16 outputs each with FP64
+//  - consumer warps computing 8 x 4 to 16 x 16 outputs each with FP64
 //    accumulation in registers over the whole K range, on the scalar FP64 pipe (DFMA, the
 //    default: 1.245 TFLOP/s at N = 16384, the GPU's FP64 rate) or on the FP64
 //    tensor cores (mma.sync.m16n8k4.f64, PHPC_FP64_PIPE=dmma: 1.089 TFLOP/s);
@@ -54,19 +54,20 @@ __device__ __forceinline__ void tile_coords(const SummaGrid& g, int t, int& rm, 
   rn = c0 + t % (c1 - c0);
 }
 
-// Square tiles of BT x BT outputs (16 or 32), warps of WM x WN. Each of the
-// SM's four quarters has its own FP64 pipe (half an FMA a clock), so both
-// tiles give every quarter a warp (FP64 tensor-core warps are at least
-// 16 x 8). Larger tiles buy nothing, since the pipe, not shared memory or L2,
-// is the limit: 64 x 64 tiles took 14.4 ms at N = 2048 against 13.8 for
-// 16 x 16, 128 x 128 tiles 895 ms at N = 8192 against 883 for 32 x 32, and a
-// call that leaves SMs idle at 64 x 64 is up to 8x slower (250 x 514 x 302:
-// 566 us against 73.6).
+// Tiles of BT x BT outputs (8: 8 x 16), warps of WM x WN. Each of the SM's
+// four quarters has its own FP64 pipe (half an FMA a clock), so all tiles give
+// every quarter a warp (8 x 4 outputs each in the 8 x 16 tile; FP64 tensor-core
+// warps are at least 16 x 8). Larger tiles buy nothing, since the pipe, not
+// shared memory or L2, is the limit: 64 x 64 tiles took 14.4 ms at N = 2048
+// against 13.8 for 16 x 16, 128 x 128 tiles 895 ms at N = 8192 against 883 for
+// 32 x 32, and a call that leaves SMs idle at 64 x 64 is up to 8x slower (250 x
+// 514 x 302: 566 us against 72.2 with 8 x 16).
 template <int BT, bool DFMA>
 struct DmmaCfg {
-  static constexpr int BM = BT, BN = BT;
+  static_assert(BT != 8 || DFMA, "an FP64 tensor-core warp has 16 rows");
+  static constexpr int BM = BT, BN = BT == 8 ? 16 : BT;
   static constexpr int WM = BT == 32 ? 16 : DFMA ? 8 : 16;
-  static constexpr int WN = BT == 32 ? 16 : 8;
+  static constexpr int WN = BT == 32 ? 16 : BT == 8 ? 4 : 8;
   static constexpr int kWarpsN = BN / WN;
   static constexpr int kConsumers = (BM / WM) * kWarpsN;
   static constexpr int kThreads = (kConsumers + 1) * 32;
@@ -93,7 +94,8 @@ __global__ void __launch_bounds__(DmmaCfg<BT, DFMA>::kThreads)
                      int64_t ldc, int M, int N, int K, int kpanel, SummaGrid grid, int stages, int* status) {
   using Cfg = DmmaCfg<BT, DFMA>;
   constexpr int BM = Cfg::BM, BN = Cfg::BN, WM = Cfg::WM, WN = Cfg::WN;
-  constexpr int NR = WM / 8, NJ = WN / 8;  // a thread's outputs: rows g + 8 r, columns 8 j + 2 tig, + 1
+  // a thread's outputs: rows g + 8 r, columns 8 j + NV tig .. + NV - 1
+  constexpr int NR = WM / 8, NJ = (WN + 7) / 8, NV = WN >= 8 ? 2 : 1;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int S = stages;  // ring depth, 2 .. kMaxStages (checked by the launcher)
@@ -156,11 +158,13 @@ __global__ void __launch_bounds__(DmmaCfg<BT, DFMA>::kThreads)
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;
-    double acc[NR][NJ][2];
+    double acc[NR][NJ][NV];
 #pragma unroll
     for (int r = 0; r < NR; ++r)
 #pragma unroll
-      for (int j = 0; j < NJ; ++j) acc[r][j][0] = acc[r][j][1] = 0.0;
+      for (int j = 0; j < NJ; ++j)
+#pragma unroll
+        for (int v = 0; v < NV; ++v) acc[r][j][v] = 0.0;
 
     for (int ks = 0; ks < ksteps; ++ks) {
       // all lanes must agree before the warp-collective mma.sync below
@@ -168,7 +172,7 @@ __global__ void __launch_bounds__(DmmaCfg<BT, DFMA>::kThreads)
       if (!ok) break;
       const double* sA = reinterpret_cast<const double*>(smem + stage * Cfg::kStageBytes);  // [BM][16]
       const double* sB = reinterpret_cast<const double*>(smem + stage * Cfg::kStageBytes + Cfg::kStageA);  // [16][BN]
-      if (DFMA) {
+      if constexpr (DFMA) {
 #pragma unroll 2
         for (int c = 0; c < kBK / 2; ++c) {
           double2 a[NR];
@@ -177,17 +181,24 @@ __global__ void __launch_bounds__(DmmaCfg<BT, DFMA>::kThreads)
             a[r] = *reinterpret_cast<const double2*>(a_chunk(sA, wm * WM + 8 * r + g, c));
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
-            double2 b[NJ];
+            double b[NJ][NV];
 #pragma unroll
-            for (int j = 0; j < NJ; ++j)
-              b[j] = *reinterpret_cast<const double2*>(&sB[(2 * c + h) * BN + wn * WN + j * 8 + 2 * tig]);
+            for (int j = 0; j < NJ; ++j) {
+              const double* src = &sB[(2 * c + h) * BN + wn * WN + j * 8 + NV * tig];
+              if constexpr (NV == 2) {
+                const double2 w = *reinterpret_cast<const double2*>(src);
+                b[j][0] = w.x;
+                b[j][1] = w.y;
+              } else {
+                b[j][0] = *src;
+              }
+            }
 #pragma unroll
             for (int r = 0; r < NR; ++r)
 #pragma unroll
-              for (int j = 0; j < NJ; ++j) {
-                acc[r][j][0] = fma(h ? a[r].y : a[r].x, b[j].x, acc[r][j][0]);
-                acc[r][j][1] = fma(h ? a[r].y : a[r].x, b[j].y, acc[r][j][1]);
-              }
+              for (int j = 0; j < NJ; ++j)
+#pragma unroll
+                for (int v = 0; v < NV; ++v) acc[r][j][v] = fma(h ? a[r].y : a[r].x, b[j][v], acc[r][j][v]);
           }
         }
       } else {
@@ -221,9 +232,10 @@ __global__ void __launch_bounds__(DmmaCfg<BT, DFMA>::kThreads)
       double* crow = C + row * ldc;
 #pragma unroll
       for (int j = 0; j < NJ; ++j) {
-        const int col = rn * BN + wn * WN + j * 8 + 2 * tig;
-        if (col < N) crow[col] += acc[r][j][0];
-        if (col + 1 < N) crow[col + 1] += acc[r][j][1];
+        const int col = rn * BN + wn * WN + j * 8 + NV * tig;
+#pragma unroll
+        for (int v = 0; v < NV; ++v)
+          if (col + v < N) crow[col + v] += acc[r][j][v];
       }
     }
   }
@@ -285,10 +297,21 @@ bool fp64_pipe_is_dfma() {
 // in 16 x 16: 1745). From 100 tiles of 32 x 32 an SM that difference is under
 // 1 % and the larger tile's fewer loads count for more (N = 3000, 58 tiles an
 // SM, K = 500: 16 7.49 ms, 32 7.55; N = 4096, 108 an SM: 110.4 and 110.15).
-// PHPC_DMMA_TILE = 16 forces the one, any other number the other.
+// Below that, 8 x 16 tiles (DFMA only; one output a thread) where they load the
+// fullest SM less, or as much with at most eight 16 x 16 tiles on it (16 / 8:
+// 64 x 2048 x 64 172.5 us, 103.1; 148 x 266 x 73 29.1, 18.8; 68 x 1384 x 1617
+// 359, 317; 582 x 1605 x 336 617, 562; 250 x 514 x 302, as much, 74.1, 72.2; but
+// N = 1024, as much with 27 tiles, 1733, 1739).
+// PHPC_DMMA_TILE = 8 or 16 forces these, any other number 32.
 int plain_tile(int m, int n, int sms) {
-  if (const char* force = getenv("PHPC_DMMA_TILE")) return atoi(force) == 16 ? 16 : 32;
-  return (int64_t)ceil_div(m, 32) * ceil_div(n, 32) >= (int64_t)100 * sms ? 32 : 16;
+  if (const char* force = getenv("PHPC_DMMA_TILE")) {
+    const int t = atoi(force);
+    return t == 16 || t == 8 ? t : 32;
+  }
+  if ((int64_t)ceil_div(m, 32) * ceil_div(n, 32) >= (int64_t)100 * sms) return 32;
+  const int64_t load16 = ((int64_t)ceil_div(m, 16) * ceil_div(n, 16) + sms - 1) / sms * 2;
+  const int64_t load8 = ((int64_t)ceil_div(m, 8) * ceil_div(n, 16) + sms - 1) / sms;
+  return load8 < load16 || (load8 == load16 && load16 <= 16) ? 8 : 16;
 }
 
 int dgemm_dmma(int m, int k, int n, const double* dA, int64_t lda, const double* dB, int64_t ldb, double* dC,
@@ -299,10 +322,14 @@ int dgemm_dmma(int m, int k, int n, const double* dA, int64_t lda, const double*
   auto launch = [&](auto tile) {
     constexpr int T = decltype(tile)::value;
     return fp64_pipe_is_dfma() ? launch_dmma<T, true>(m, k, n, dA, lda, dB, ldb, dC, ldc, gw, gh, kpanel, stream)
-                               : launch_dmma<T, false>(m, k, n, dA, lda, dB, ldb, dC, ldc, gw, gh, kpanel, stream);
+                               : launch_dmma<T == 8 ? 16 : T, false>(m, k, n, dA, lda, dB, ldb, dC, ldc, gw, gh,
+                                                                     kpanel, stream);
   };
-  return plain_tile(m, n, dev->sm_count) == 16 ? launch(std::integral_constant<int, 16>())
-                                                : launch(std::integral_constant<int, 32>());
+  switch (plain_tile(m, n, dev->sm_count)) {
+    case 8: return launch(std::integral_constant<int, 8>());
+    case 16: return launch(std::integral_constant<int, 16>());
+    default: return launch(std::integral_constant<int, 32>());
+  }
 }
 
 }  // namespace phpc

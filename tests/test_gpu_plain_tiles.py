@@ -1,4 +1,4 @@
-"""The plain FP64 GEMM's tiles (16 x 16 and 32 x 32) on both pipes.
+"""The plain FP64 GEMM's tiles (8 x 16, 16 x 16 and 32 x 32) on both pipes.
 
 Every output is summed over k in increasing order with one rounding per FMA
 and added into C once, whatever the tile, pipe or SUMMA grid, so all variants
@@ -9,7 +9,7 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("m,k,n", [(1, 1, 1), (15, 16, 17), (16, 17, 16), (33, 15, 31), (65, 300, 40), (250, 514, 302)])
+@pytest.mark.parametrize("m,k,n", [(1, 1, 1), (15, 16, 17), (16, 17, 16), (33, 15, 31), (65, 300, 40), (250, 514, 302), (68, 200, 1617)])
 @pytest.mark.parametrize("gw,gh", [(1, 1), (3, 2), (64, 64)])
 def test_tiles_pipes_and_grids_same_bits(phpc, torch_cuda, monkeypatch, m, k, n, gw, gh):
     torch = torch_cuda
@@ -19,7 +19,7 @@ def test_tiles_pipes_and_grids_same_bits(phpc, torch_cuda, monkeypatch, m, k, n,
     B = torch.randn((k, ldb), dtype=torch.float64, device="cuda", generator=g)
     C0 = torch.randn((m, ldc), dtype=torch.float64, device="cuda", generator=g)
     outs = {}
-    for tile in ("16", "32", None):
+    for tile in ("8", "16", "32", None):
         for pipe in ("dfma", "dmma"):
             monkeypatch.setenv("PHPC_FP64_PIPE", pipe)
             if tile:
