@@ -161,6 +161,42 @@ __global__ void g_scan_cols_part_kernel(const GSplitProb* __restrict__ P, int co
   if (nf) record_error(status, PHPC_ERR_NONFINITE);
 }
 
+// The same sums for a batch of few units: a block takes 32 units, warp w rows
+// 32 w .. + 31 of each, and warp 0 merges the eight slices in order, so that a
+// chain is 32 rows instead of 256.
+__global__ void __launch_bounds__(256) g_scan_cols_slices_kernel(const GSplitProb* __restrict__ P, int count,
+                                                                 int total_units, int* status) {
+  __shared__ int se[8][32];
+  __shared__ float ss[8][32];
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  const int u = blockIdx.x * 32 + l;
+  const int v = min(u, total_units - 1);  // whole warps below
+  const GSplitProb& p = P[locate_warp(P, count, v, [](const GSplitProb& q) { return q.cunit_start; })];
+  const int unit = v - p.cunit_start;
+  const int64_t col = unit % p.n;
+  const int chunk = unit / p.n, k0 = chunk * kNormChunk + w * kNormSlice;
+  bool nf = false;
+  NormAcc acc;
+  if (k0 < p.k) norm_col_slice(p.B, p.ldb, col, k0, p.k, acc, nf);
+  se[w][l] = acc.e;
+  ss[w][l] = acc.s;
+  if (nf) record_error(status, PHPC_ERR_NONFINITE);
+  __syncthreads();
+  if (w != 0 || u >= total_units) return;
+  acc = NormAcc{};
+#pragma unroll
+  for (int q = 0; q < 8; ++q) norm_merge(acc, NormAcc{se[q][l], ss[q][l]});
+  p.pe[(int64_t)chunk * p.n + col] = acc.e;
+  p.ps[(int64_t)chunk * p.n + col] = acc.s;
+}
+
+// Which: below 160 units an SM (5 warps of the first form) the chains' latency
+// is what counts. A whole batch, thread per unit / slices: 8 problems of 32 to
+// 300 (1676 units) 43.4 us, 35.8; 64 of 16 to 256 (5542) 66.7, 58.3; 16 of 64 to
+// 2048 (15816) 219, 211; but 512 of 16 to 256 (45253) 292, 299, where rows
+// beyond K idle most slices, and 200 of 32 to 1000 (98267) 727, 738.
+constexpr int kSliceUnitsPerSm = 160;
+
 // Part 2: one thread per column merges its chunks in order: eb[j], bb[j].
 __global__ void g_scan_cols_merge_kernel(const GSplitProb* __restrict__ P, int count, int total_cols,
                                          const __grid_constant__ ModTable T) {
@@ -461,6 +497,8 @@ int prepare_grouped_gemm(const DeviceInfo* dev) {
 
 int run_grouped(const phpc_grouped_plan* pl, cudaStream_t stream) {
   int* status = device_status_ptr();
+  const DeviceInfo* dev = current_device();
+  if (!dev) return PHPC_ERR_CUDA;
   const bool modular = pl->moduli > 0;
   if (pl->total_rows > 0) {
     if (modular) {
@@ -470,8 +508,12 @@ int run_grouped(const phpc_grouped_plan* pl, cudaStream_t stream) {
       if (!side || !stream_fork(stream, side)) side = stream;
       g_scan_rows_grid_kernel<<<ceil_div(pl->total_rows, 8), 256, 0, stream>>>(pl->d_split, pl->count,
                                                                                pl->total_rows, pl->mods, status);
-      g_scan_cols_part_kernel<<<ceil_div(pl->total_cunits, 128), 128, 0, side>>>(pl->d_split, pl->count,
-                                                                                 pl->total_cunits, status);
+      if (pl->total_cunits < kSliceUnitsPerSm * dev->sm_count)
+        g_scan_cols_slices_kernel<<<ceil_div(pl->total_cunits, 32), 256, 0, side>>>(pl->d_split, pl->count,
+                                                                                    pl->total_cunits, status);
+      else
+        g_scan_cols_part_kernel<<<ceil_div(pl->total_cunits, 128), 128, 0, side>>>(pl->d_split, pl->count,
+                                                                                   pl->total_cunits, status);
       g_scan_cols_merge_kernel<<<ceil_div(pl->total_cols, 256), 256, 0, side>>>(pl->d_split, pl->count,
                                                                                 pl->total_cols, pl->mods);
       with_crt_moduli(pl->mods.n, [&](auto nm) {
