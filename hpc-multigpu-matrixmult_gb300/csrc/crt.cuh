@@ -1,6 +1,5 @@
-// Chinese-remainder reconstruction of the modular Ozaki scheme, shared by
-// the standalone CRT kernel (ozaki2.cu) and the residue GEMM's fused
-// epilogue (tc_gemm.cuh).
+// Chinese-remainder reconstruction of the modular Ozaki scheme, shared by the
+// CRT kernels of the single call (ozaki2.cu) and the batch (grouped.cu).
 #pragma once
 
 #include <cstdint>

@@ -7,9 +7,10 @@
 // whole batch once:
 //  - a device table with one record per problem and the prefix sums of its
 //    rows, columns, split blocks and output tiles, plus two TMA descriptors
-//    per problem (A digit planes, B digit planes) and a table of the output
-//    tiles (problem, tile row and column, K-steps), written into the head of
-//    the caller's workspace;
+//    per problem (A planes, B planes; the modular scheme a third, for the
+//    stores into its residue planes) and a table of the output tiles (problem,
+//    tile row and column, K-steps), written into the head of the caller's
+//    workspace;
 //  - five kernels cover the batch (six launches: the column scan's reset):
 //    exponent scans of all rows, of all columns, digit splits of all rows,
 //    of all column blocks, and the
@@ -18,10 +19,11 @@
 //    table);
 //  - phpc_grouped_graph_launch captures those five launches once into a CUDA
 //    graph and replays it.
-// A modular-scheme plan (phpc_grouped_modular_plan_create) has six kernels:
-// the two scans, residue splits of all rows and of all column blocks, the
-// persistent residue GEMM over all tiles (each tile's residues go to its
-// problem's planes), and the CRT of all rows; every problem uses the plan's
+// A modular-scheme plan (phpc_grouped_modular_plan_create) has seven kernels:
+// the row scan, the column scan and the merge of its chunks, residue splits of
+// all rows and of all column blocks, the persistent residue GEMM over all
+// (tile, modulus) units (each tile's residues go to its problem's planes), and
+// the CRT of all rows; every problem uses the plan's
 // moduli and the grid width of its own K. Its residue splits and CRT find a
 // block's problem in lookup tables the plan also writes.
 #include <cuda.h>
