@@ -312,8 +312,16 @@ __global__ void __launch_bounds__(32 * kCrtBlockUnits, crt_min_blocks(NMOD, true
   const int u = blockIdx.x * kCrtBlockUnits + (threadIdx.x >> 5);
   if (u >= total_units) return;
   int pi = first[blockIdx.x];
-  while (pi + 1 < count && P[pi + 1].crt_unit_start <= u) ++pi;
-  const GSplitProb& p = P[pi];
+  int next = P[min(pi + 1, count - 1)].crt_unit_start;
+  // The record comes with the load of next, not after it (a warp rarely walks
+  // on): one L2 latency less in front of the planes' loads, the 512-problem
+  // batch 6824 -> 6786 us. (In the row split it made no difference.)
+  GSplitProb p = P[pi];
+  while (pi + 1 < count && next <= u) {
+    ++pi;
+    p = P[pi];
+    next = P[min(pi + 1, count - 1)].crt_unit_start;
+  }
   const int64_t gpr = (p.n + kCrtCols - 1) / kCrtCols;  // groups per row
   const int64_t g = (int64_t)(u - p.crt_unit_start) * 32 + (threadIdx.x & 31);
   const int64_t groups = p.m * gpr;
