@@ -145,7 +145,7 @@ int ksplit_clusters(int split, const DeviceInfo* dev) {
 // unsplit / chosen / one more: 1000 x 777 x 1530 (48 tiles) 49.4 us, 37.1
 // with 2, 50 with 3 (144 CTAs in clusters of 3 do not fit at once); N = 1024
 // (32 tiles) 53.5, 32.2 with 4, 47.5 with 5; 700 x 3000 x 900 117, 48.3 with 5,
-// 66 with 8; 128 x 4096 x 512 140, 41 with 8. Below 48 steps (K <= 448) there
+// 66 with 8; 128 x 4096 x 512 140, 41 with 8. Below kF32SplitSteps (K <= 448) there
 // is little to share and the shares' additions would cost accuracy; from there
 // the error is 0.43 to 0.7 of the unsplit one (1000 x 777 x 1530: 2.1e-7
 // against 3.7e-7), since a share flushes its accumulator twice as often.
@@ -156,7 +156,7 @@ int f32_ksplit(int m, int n, int steps, const DeviceInfo* dev) {
   if (env && atoi(env) >= 1 && atoi(env) <= kMaxKsplit) return std::min(atoi(env), steps);
   const int64_t tiles = (int64_t)ceil_div(m, kTcBM) * ceil_div(n, 256);
   for (int s = kMaxKsplit; s > 1; --s)
-    if (tiles * s <= dev->sm_count && steps >= 48 && steps / s >= 4 && tiles <= ksplit_clusters<BN, kF32>(s, dev)) return s;
+    if (tiles * s <= dev->sm_count && steps >= kF32SplitSteps && steps / s >= 4 && tiles <= ksplit_clusters<BN, kF32>(s, dev)) return s;
   return 1;
 }
 

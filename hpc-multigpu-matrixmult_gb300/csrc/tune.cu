@@ -238,6 +238,25 @@ int default_grouped_stages(const phpc_gemm_problem* problems, int count) {
   return 0;
 }
 
+namespace {
+
+// Where the 3xBF16 GEMM takes 128-wide tiles although its table entry says
+// 256: a call that K is not split for and whose 128 x 128 tiles all run at
+// once takes as long as one tile, half of it the C += AB of a warp's columns,
+// 32 at a time; and columns beyond n <= 128 are only padding. Replayed graphs,
+// 256 / 128: 500 x 94 x 500 18.5 us, 12.5; 1000 x 300 x 1000 24.1, 18.4; 1000 x
+// 440 x 2000 (128 tiles) 28.8, 22.7; 584 x 495 x 84 15.8, 12.5. With a second
+// wave, or with K split, the wide tile's fewer operand bytes count: 4868 x 216 x
+// 605 (195 tiles) 28.4, 30.7; 1000 x 777 x 1530 28.4, 43.3.
+bool f32_narrow(int m, int k, int n) {
+  if (n <= 128) return true;
+  const DeviceInfo* dev = current_device();
+  return dev && 6 * ceil_div(k, 64) < kF32SplitSteps &&
+         (int64_t)ceil_div(m, 128) * ceil_div(n, 128) <= dev->sm_count;
+}
+
+}  // namespace
+
 F32Tune default_f32(int m, int k, int n) {
   F32Tune t{256, 8, 0};
   std::call_once(g_once, load_table);
@@ -247,6 +266,7 @@ F32Tune default_f32(int m, int k, int n) {
       t = {e.bn, e.group_rows, e.stages};
       break;
     }
+  if (t.bn == 256 && f32_narrow(m, k, n)) t.bn = 128;
   if (const char* env = getenv("PHPC_F32_BN"))
     if (atoi(env) == 128 || atoi(env) == 256) t.bn = atoi(env);
   if (const char* env = getenv("PHPC_GROUP_ROWS"))
