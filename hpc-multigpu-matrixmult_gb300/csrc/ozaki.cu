@@ -181,6 +181,13 @@ int residue_ksplit(int64_t units, int steps, const DeviceInfo* dev) {
 
 }  // namespace
 
+// Whether the 3xBF16 GEMM splits K and all its 128-wide tiles would run at
+// once with that split too.
+bool f32_narrow_split(int m, int k, int n, const DeviceInfo* dev) {
+  const int split = f32_ksplit<256>(m, n, 6 * ceil_div(k, kTcBK), dev);
+  return split > 1 && (int64_t)ceil_div(m, kTcBM) * ceil_div(n, 128) <= ksplit_clusters<128, kF32>(split, dev);
+}
+
 // Launches the tcgen05 slice GEMM over bf16 planes (shared with the 3xBF16
 // and modular paths).
 template <int BN, int MODE>

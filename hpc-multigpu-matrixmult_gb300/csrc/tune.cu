@@ -245,14 +245,18 @@ namespace {
 // once takes as long as one tile, half of it the C += AB of a warp's columns,
 // 32 at a time; and columns beyond n <= 128 are only padding. Replayed graphs,
 // 256 / 128: 500 x 94 x 500 18.5 us, 12.5; 1000 x 300 x 1000 24.1, 18.4; 1000 x
-// 440 x 2000 (128 tiles) 28.8, 22.7; 584 x 495 x 84 15.8, 12.5. With a second
-// wave, or with K split, the wide tile's fewer operand bytes count: 4868 x 216 x
-// 605 (195 tiles) 28.4, 30.7; 1000 x 777 x 1530 28.4, 43.3.
+// 440 x 2000 (128 tiles) 28.8, 22.7; 584 x 495 x 84 15.8, 12.5. The same holds
+// with K split, whose shares then exchange half as much, while the clusters of
+// the narrow tiles still run at once (calls: 132 x 3857 x 268, 6 clusters of 8,
+// 35.0, 30.0; 611 x 2534 x 279, 15 clusters, 31.2, 26.4; but 16: 250 x 600 x 900
+// 20.8, 27.1). With a second wave the wide tile's fewer operand bytes count:
+// 4868 x 216 x 605 (195 tiles) 28.4, 30.7; 1000 x 777 x 1530 28.4, 43.3.
 bool f32_narrow(int m, int k, int n) {
   if (n <= 128) return true;
   const DeviceInfo* dev = current_device();
-  return dev && 6 * ceil_div(k, 64) < kF32SplitSteps &&
-         (int64_t)ceil_div(m, 128) * ceil_div(n, 128) <= dev->sm_count;
+  if (!dev) return false;
+  if (6 * ceil_div(k, 64) < kF32SplitSteps) return (int64_t)ceil_div(m, 128) * ceil_div(n, 128) <= dev->sm_count;
+  return f32_narrow_split(m, k, n, dev);
 }
 
 }  // namespace

@@ -30,10 +30,11 @@ def test_exact_update(phpc, torch_cuda, monkeypatch, bn, m, k, n):
         assert torch.equal(C[:, n:], C0[:, n:]) and torch.equal(C[m], C0[m])  # nothing outside the block
 
 
-@pytest.mark.parametrize("m,k,n", [(300, 94, 500), (1500, 448, 1500), (2100, 448, 1500), (129, 500, 128), (129, 500, 129)])
+@pytest.mark.parametrize("m,k,n", [(300, 94, 500), (1500, 448, 1500), (2100, 448, 1500), (129, 500, 128), (129, 500, 129),
+                                   (132, 1200, 268), (611, 900, 279), (250, 600, 900)])
 def test_tile_width_same_bits(phpc, torch_cuda, monkeypatch, m, k, n):
     """Both sides of the rules for 128-wide tiles (tiles that all run at once
-    with K unsplit, n <= 128): the bits of the 256-wide tile."""
+    with K unsplit or split, n <= 128): the bits of the 256-wide tile."""
     torch = torch_cuda
     g = torch.Generator(device="cuda").manual_seed(m + k + n)
     A = torch.randn((m, k), device="cuda", generator=g)
