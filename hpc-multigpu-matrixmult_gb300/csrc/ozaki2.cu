@@ -535,7 +535,7 @@ extern "C" int phpc_ozaki2_multiply_dev(int m, int k, int n, int moduli, void* w
   int rc = ozaki2_args(m, k, n, moduli, false, nullptr, 0, false, nullptr, 0, false, nullptr, 0);
   if (rc == PHPC_OK && m > 0 && n > 0 && k > 0)
     rc = phpc::ozaki2_multiply(m, k, n, moduli, workspace, workspace_bytes, static_cast<cudaStream_t>(stream),
-                               phpc::default_bn(m, k, n));
+                               phpc::modular_bn(m, k, n, moduli));
   phpc::set_last_error(rc);
   return rc;
 }
@@ -556,7 +556,7 @@ extern "C" int phpc_dgemm_ozaki2_dev(int m, int k, int n, const double* dA, int6
   int rc = ozaki2_args(m, k, n, moduli, true, dA, lda, true, dB, ldb, true, dC, ldc);
   if (rc == PHPC_OK && m > 0 && n > 0 && k > 0)
     rc = phpc::dgemm_ozaki2(m, k, n, dA, lda, dB, ldb, dC, ldc, moduli, workspace, workspace_bytes,
-                            static_cast<cudaStream_t>(stream), phpc::default_bn(m, k, n));
+                            static_cast<cudaStream_t>(stream), phpc::modular_bn(m, k, n, moduli));
   phpc::set_last_error(rc);
   return rc;
 }

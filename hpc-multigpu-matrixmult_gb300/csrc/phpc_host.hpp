@@ -145,6 +145,7 @@ int default_slices(int m, int k, int n);
 // scheme (default_slices slices).
 int default_moduli(int m, int k, int n);
 int default_bn(int m, int k, int n);
+int modular_bn(int m, int k, int n, int moduli);
 int default_grouped_bn(const phpc_gemm_problem* problems, int count);
 int default_group_rows(int m, int k, int n);
 int default_cluster(int m, int k, int n);

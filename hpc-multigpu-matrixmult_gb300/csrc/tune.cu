@@ -153,6 +153,22 @@ int default_bn(int m, int k, int n) {
   return 256;
 }
 
+// Tile width of a modular call's residue GEMM: default_bn, but 128 where the
+// table says 256 and the (128-wide tile, modulus) units all run at once, so
+// that the call waits for one unit's drain and stores of half the columns, or
+// where columns beyond n <= 128 would only be padding. Whole calls, 256 / 128:
+// 86 x 1343 x 615 33.5 us, 31.4; 235 x 3167 x 169 48.0, 45.6; 124 x 2991 x 1317
+// (143 units) 89.9, 87.1; 336 x 4001 x 72 50.4, 47.1; 8000 x 1000 x 100 143, 137;
+// N = 256 17.8, 16.4 as a graph. With more units than SMs the wide tile's fewer
+// operand bytes count: GEMM of 664 x 1420 x 668 22.8, 35.0. Exact either way.
+int modular_bn(int m, int k, int n, int moduli) {
+  const int bn = default_bn(m, k, n);
+  if (bn == 128 || getenv("PHPC_OZAKI_BN")) return bn;
+  if (n <= 128) return 128;
+  const DeviceInfo* dev = current_device();
+  return dev && (int64_t)ceil_div(m, 128) * ceil_div(n, 128) * moduli <= dev->sm_count ? 128 : bn;
+}
+
 namespace {
 
 // Whether CTA pairs suit the shape where the table has them. A pair stages 32

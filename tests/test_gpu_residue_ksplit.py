@@ -34,3 +34,26 @@ def test_same_bits(phpc, torch_cuda, monkeypatch, bn, moduli, m, k, n):
         assert torch.equal(C, ref), split
     assert torch.equal(ref[:, n:], C0[:, n:]) and torch.equal(ref[m], C0[m])
     assert not torch.equal(ref[:m, :n], C0[:m, :n])
+
+
+@pytest.mark.parametrize("m,k,n", [(128, 70, 128), (300, 300, 129), (124, 600, 1317), (600, 600, 400), (3000, 520, 100)])
+def test_tile_width_same_bits(phpc, torch_cuda, monkeypatch, m, k, n):
+    """Both sides of the rule for 128-wide tiles (n <= 128, units that all run
+    at once): the bits of the 256-wide tile."""
+    torch = torch_cuda
+    g = torch.Generator(device="cuda").manual_seed(m + k + n)
+    A = torch.randn((m, k), dtype=torch.float64, device="cuda", generator=g)
+    B = torch.randn((k, n), dtype=torch.float64, device="cuda", generator=g)
+    C0 = torch.randn((m, n), dtype=torch.float64, device="cuda", generator=g)
+    size = phpc.ozaki2_workspace_bytes(m, k, n, 13)
+    W = torch.empty(size, dtype=torch.uint8, device="cuda")
+    outs = []
+    for bn in (None, "256", "128"):
+        if bn:
+            monkeypatch.setenv("PHPC_OZAKI_BN", bn)
+        C = C0.clone()
+        phpc.dgemm_ozaki2_dev(m, k, n, A, k, B, n, C, n, 13, W, size)
+        outs.append(C)
+    torch.cuda.synchronize()
+    assert phpc.device_status() == 0
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
