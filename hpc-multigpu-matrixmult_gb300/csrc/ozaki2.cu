@@ -115,10 +115,9 @@ __global__ void __launch_bounds__(kPrepThreads) scan_kernel(const PrepRows a, co
 
 // Column scan, part 2: a block merges the chunks of 32 columns, warp p those
 // numbered p, p + 8, ..., into eb[j] and bb[j].
-__global__ void __launch_bounds__(256) scan_cols_merge_kernel(int K, int N, int64_t ldpart,
-                                                              const int* __restrict__ pe,
-                                                              const float* __restrict__ ps, int* __restrict__ eb,
-                                                              int* __restrict__ bb, float logT) {
+// (No __restrict__ on what the scan writes: see launch_dependent.)
+__global__ void __launch_bounds__(256) scan_cols_merge_kernel(int K, int N, int64_t ldpart, const int* pe,
+                                                              const float* ps, int* eb, int* bb, float logT) {
   __shared__ int se[8][32];
   __shared__ float ss[8][32];
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
@@ -200,12 +199,12 @@ __global__ void __launch_bounds__(kPrepThreads, 4)
                           b.plane_stride, tile);
 }
 
-// C[i][j] += C_int * 2^(ea[i] - ba[i] + eb[j] - bb[j]), C_int recovered from the residues.
+// C[i][j] += C_int * 2^(ea[i] - ba[i] + eb[j] - bb[j]), C_int recovered from
+// the residues. (No __restrict__ on what earlier grids write: see launch_dependent.)
 template <int NMOD>
 __global__ void __launch_bounds__(128, crt_min_blocks(NMOD, false))
-    crt_kernel(const uint16_t* __restrict__ R, int64_t ldr, int64_t rplane, int M, int N, const int* __restrict__ ea,
-               const int* __restrict__ ba, const int* __restrict__ eb, const int* __restrict__ bb,
-               const __grid_constant__ ModTable T, double* __restrict__ C, int64_t ldc) {
+    crt_kernel(const uint16_t* R, int64_t ldr, int64_t rplane, int M, int N, const int* ea, const int* ba,
+               const int* eb, const int* bb, const __grid_constant__ ModTable T, double* C, int64_t ldc) {
   const int64_t row = blockIdx.x;
   const int64_t c0 = ((int64_t)blockIdx.y * blockDim.x + threadIdx.x) * kCrtCols;
   pdl_wait();

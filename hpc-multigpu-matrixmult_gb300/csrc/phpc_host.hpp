@@ -37,7 +37,10 @@ inline int ceil_div(int64_t a, int64_t b) { return static_cast<int>((a + b - 1) 
 // Launches a kernel; with `dependent` it may come up while the kernel before it
 // on the stream finishes (programmatic dependent launch: the kernel calls
 // pdl_wait before it touches global memory). Only for a kernel that directly
-// follows one of this library's own on the stream.
+// follows one of this library's own on the stream. Such a kernel takes no
+// __restrict__ pointers: its inputs are still being written when it starts, and
+// the qualifier would let the compiler read them through the non-coherent path
+// or ahead of the wait.
 template <class... P, class... A>
 cudaError_t launch_dependent(bool dependent, void (*kern)(P...), dim3 grid, dim3 block, size_t smem,
                              cudaStream_t stream, A&&... args) {
