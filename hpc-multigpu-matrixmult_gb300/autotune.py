@@ -12,7 +12,8 @@ sampled rows, for two input classes: uniform [-1, 1) and wide exponents
 (u * 2^e, e uniform in [-20, 20]). A configuration qualifies when both errors
 are below target / margin; the fastest qualifying configuration wins, and
 then the pipeline depth (K-stages of the tcgen05 shared-memory ring, 2 up to
-the deepest that fits) is swept for it. For the grouped call it picks BN and
+the deepest that fits) is swept for it. The digit scheme's fastest tile width
+and grouping at each size go into "digits" entries. For the grouped call it picks BN and
 the stages on the batching workload (512 problems, modular plan with
 --grouped-moduli moduli); for the 3xBF16 FP32 GEMM the tile width, raster and
 stages on the rectangular workload (M = 32768, N = 8192, K = 4096, FP32
@@ -65,7 +66,7 @@ def main() -> int:
     sizes = [n for n in (int(x) for x in a.sizes.split(",")) if n <= a.max_n]
     schemes = [("moduli", int(x)) for x in a.moduli.split(",") if x] + \
               [("slices", int(x)) for x in a.slices.split(",") if x]
-    table, report = [], []
+    table, report, digits = [], [], []
 
     clusters = [int(x) for x in a.clusters.split(",")]
 
@@ -153,6 +154,9 @@ def main() -> int:
         if not cands:
             raise SystemExit(f"no configuration meets {a.target} / {a.margin} at N={n}")
         best, run, W = min(cands, key=lambda c: c[0]["ms"])
+        # the digit scheme's own tile width and cluster, which the winner's entry also governs
+        mine = [r for r in report if r.get("n") == n and r.get("moduli") == 0]
+        digits.append(min(mine, key=lambda r: r["ms"]) if mine else None)
         # pipeline depth of the winner: 2 .. the deepest ring that fits (0 = deepest)
         A, B, _, _ = classes["wide"]
         deepest = max_stages(best["bn"], best["cluster"])
@@ -281,6 +285,11 @@ def main() -> int:
         bound = int((b["n"] ** 3 * nxt ** 3) ** 0.5) if nxt else 2 ** 62
         lines.append(f"# N={b['n']}: {b['ms']} ms, {b['tflops']} TFLOP/s, err {b['err']}")
         lines.append(f"{bound} {b['slices']} {b['bn']} {b['group_rows']} {b['cluster']} {b['moduli']} {b['stages']}")
+    for i, (b, d) in enumerate(zip(table, digits)):
+        if d is not None:
+            bound = int((b["n"] ** 3 * table[i + 1]["n"] ** 3) ** 0.5) if i + 1 < len(table) else 2 ** 62
+            lines.append(f"# digits N={b['n']}: {d['ms']} ms")
+            lines.append(f"digits {bound} {d['bn']} {d['cluster']}")
     lines.append(f"# grouped ({a.grouped_count} problems, {a.grouped_moduli} moduli): bn {grouped_bn}, stages "
                  f"{grouped_stages}, {round(best_ms, 3) if best_ms else None} ms")
     lines.append(f"grouped {2 ** 62} 7 {grouped_bn} {grouped_stages}")

@@ -181,7 +181,7 @@ int host_gemm(Method method, const double* a, int lda, const double* b, int ldb,
         if (method == kDmma) {
           rc = dgemm_dmma(m, k, n, r.dA, dlda, r.dB, dldb, r.dC, dldc, gw, gh, 256, s0);
         } else {
-          rc = ozaki_multiply(m, k, n, r.dC, dldc, slices, r.ws, ws_bytes, s0, default_bn(m, k, n));
+          rc = ozaki_multiply(m, k, n, r.dC, dldc, slices, r.ws, ws_bytes, s0, digit_bn(m, k, n));
         }
       }
     }

@@ -209,7 +209,7 @@ int launch_tc_slice_gemm(const void* planesA, const void* planesB, int nplanesA,
             ck = opt.cfg_k > 0 ? opt.cfg_k : k;
   // the 3xBF16 GEMM has its own table entries ("f32") and runs on single CTAs
   const F32Tune f32 = MODE == kF32 ? default_f32(cm, ck, cn) : F32Tune{};
-  const int cluster = MODE == kF32 ? 1 : default_cluster(cm, ck, cn);
+  const int cluster = MODE == kF32 ? 1 : MODE == kOzaki ? digit_cluster(cm, ck, cn) : default_cluster(cm, ck, cn);
   const uint32_t bB[3] = {kTcBK, (uint32_t)(BN / cluster), 1};  // with a 2-CTA cluster each CTA loads half of B
   if (!encode_tiled(&tmA, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, planesA, dA, sA, bA, CU_TENSOR_MAP_SWIZZLE_128B) ||
       !encode_tiled(&tmB, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, planesB, dB, sB, bB, CU_TENSOR_MAP_SWIZZLE_128B))
@@ -417,7 +417,7 @@ extern "C" int phpc_ozaki_multiply_dev(int m, int k, int n, double* dC, int64_t 
       rc = PHPC_ERR_ARG;
     else
       rc = ozaki_multiply(m, k, n, dC, ldc, slices, workspace, workspace_bytes, static_cast<cudaStream_t>(stream),
-                          default_bn(m, k, n));
+                          digit_bn(m, k, n));
   }
   set_last_error(rc);
   return rc;
@@ -436,7 +436,7 @@ extern "C" int phpc_dgemm_ozaki_dev(int m, int k, int n, const double* dA, int64
     rc = PHPC_ERR_ARG;
   } else {
     rc = dgemm_ozaki(m, k, n, dA, lda, dB, ldb, dC, ldc, slices, workspace, workspace_bytes,
-                     static_cast<cudaStream_t>(stream), default_bn(m, k, n));
+                     static_cast<cudaStream_t>(stream), digit_bn(m, k, n));
   }
   set_last_error(rc);
   return rc;
@@ -515,7 +515,7 @@ extern "C" int phpc_dgemm_ozaki_noalloc_dev(int m, int k, int n, const double* d
     rc = noalloc_scratch(&ws);
     if (rc == PHPC_OK)
       rc = dgemm_ozaki(m, k, n, dA, lda, dB, ldb, dC, ldc, slices, ws, (size_t)PHPC_NOALLOC_SCRATCH_BYTES,
-                       static_cast<cudaStream_t>(stream), default_bn(m, k, n));
+                       static_cast<cudaStream_t>(stream), digit_bn(m, k, n));
   }
   set_last_error(rc);
   return rc;

@@ -123,7 +123,7 @@ int accurate_panel(phpc_panels* p, int s, int k) {
   if (nonfinite) PHPC_CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(int), p->comp));
   rc = mark(p);
   if (rc != PHPC_OK) return rc;
-  const int bn = default_bn(m, k, n);
+  const int bn = nmod ? default_bn(m, k, n) : digit_bn(m, k, n);
   if (nonfinite)
     rc = dgemm_dmma(m, k, n, p->dA[s], p->dlda, p->dB[s], p->dldb, p->dC, p->dldc, 1, 1, 256, p->comp);
   else if (!nmod)

@@ -148,6 +148,8 @@ int default_slices(int m, int k, int n);
 // scheme (default_slices slices).
 int default_moduli(int m, int k, int n);
 int default_bn(int m, int k, int n);
+int digit_bn(int m, int k, int n);       // the digit GEMM's tile width
+int digit_cluster(int m, int k, int n);  // and CTAs per cluster
 int modular_bn(int m, int k, int n, int moduli);
 int default_grouped_bn(const phpc_gemm_problem* problems, int count);
 int default_group_rows(int m, int k, int n);

@@ -44,12 +44,18 @@ struct PlainEntry {
   long long max_mnk;
   int stages;
 };
+// "digits max_mnk bn cluster": the digit GEMM of single problems.
+struct DigitEntry {
+  long long max_mnk;
+  int bn, cluster;
+};
 
 std::once_flag g_once;
 std::vector<TuneEntry> g_table;    // single-problem entries
 std::vector<TuneEntry> g_grouped;  // grouped-call entries (lines starting with "grouped")
 std::vector<F32Entry> g_f32;       // 3xBF16 entries (lines starting with "f32")
 std::vector<PlainEntry> g_plain;   // plain FP64 entries (lines starting with "plain")
+std::vector<DigitEntry> g_digits;  // digit-scheme entries (lines starting with "digits")
 
 std::string library_dir() {
   Dl_info info;
@@ -64,8 +70,9 @@ std::string library_dir() {
 // Table format (text): one entry per line, "max_mnk slices bn [group_rows
 // [cluster [moduli [stages]]]]" for single problems, "grouped max_mean_mnk
 // slices bn [stages]" for grouped calls, "f32 max_mnk bn group_rows stages"
-// for the 3xBF16 GEMM and "plain max_mnk stages" for the plain FP64 GEMM;
-// '#' starts a comment line; the first entry whose max_mnk covers the
+// for the 3xBF16 GEMM, "plain max_mnk stages" for the plain FP64 GEMM and
+// "digits max_mnk bn cluster" where the digit GEMM's choice is not that of the
+// single-problem entry; '#' starts a comment line; the first entry whose max_mnk covers the
 // problem applies. Written by autotune.py.
 void load_table() {
   const char* env = getenv("PHPC_TUNE_TABLE");
@@ -97,6 +104,13 @@ void load_table() {
         g_plain.push_back(pe);
       continue;
     }
+    if (strncmp(line, "digits", 6) == 0) {
+      DigitEntry de{};
+      if (sscanf(line + 6, "%lld %d %d", &de.max_mnk, &de.bn, &de.cluster) == 3 && (de.bn == 128 || de.bn == 256) &&
+          (de.cluster == 1 || de.cluster == 2))
+        g_digits.push_back(de);
+      continue;
+    }
     const int got = sscanf(line, "%lld %d %d %d %d %d %d", &e.max_mnk, &e.slices, &e.bn, &e.group_rows, &e.cluster,
                            &e.moduli, &e.stages);
     if (got >= 3 && e.slices >= 2 && e.slices <= 8 && (e.bn == 128 || e.bn == 256)) {
@@ -116,6 +130,31 @@ const TuneEntry* lookup(int m, int k, int n) {
   for (const TuneEntry& e : g_table)
     if (mnk <= e.max_mnk) return &e;
   return nullptr;
+}
+
+// Tile width and CTAs per cluster of the digit GEMM (0: not set): the first
+// "digits" entry that covers the problem, else its single-problem entry. The
+// two schemes part where tiles are few: the residue GEMM has a CTA per (tile,
+// modulus), the digit GEMM one per tile, so N = 512 to 1448 wants twice as many
+// tiles half as wide.
+DigitEntry digit_entry(int m, int k, int n) {
+  const TuneEntry* e = lookup(m, k, n);
+  const long long mnk = (long long)m * n * k;
+  for (const DigitEntry& d : g_digits)
+    if (mnk <= d.max_mnk) return d;
+  return e ? DigitEntry{e->max_mnk, e->bn, e->cluster} : DigitEntry{};
+}
+
+// The tile width PHPC_OZAKI_BN names (0: none), the cluster PHPC_CLUSTER names.
+int env_bn() {
+  const char* env = getenv("PHPC_OZAKI_BN");
+  const int b = env ? atoi(env) : 0;
+  return b == 128 || b == 256 ? b : 0;
+}
+int env_cluster() {
+  const char* env = getenv("PHPC_CLUSTER");
+  const int c = env ? atoi(env) : 0;
+  return c == 1 || c == 2 ? c : 0;
 }
 
 }  // namespace
@@ -144,13 +183,20 @@ int default_moduli(int m, int k, int n) {
 }
 
 int default_bn(int m, int k, int n) {
-  const char* env = getenv("PHPC_OZAKI_BN");
-  if (env) {
-    const int b = atoi(env);
-    if (b == 128 || b == 256) return b;
-  }
+  if (const int b = env_bn()) return b;
   if (const TuneEntry* e = lookup(m, k, n)) return e->bn;
   return 256;
+}
+
+int digit_bn(int m, int k, int n) {
+  if (const int b = env_bn()) return b;
+  const DigitEntry d = digit_entry(m, k, n);
+  return d.bn ? d.bn : 256;
+}
+
+int digit_cluster(int m, int k, int n) {
+  if (const int c = env_cluster()) return c;
+  return digit_entry(m, k, n).cluster == 2 ? 2 : 1;
 }
 
 // Tile width of a modular call's residue GEMM: default_bn, but 128 where the
@@ -191,13 +237,12 @@ bool pairs_fit(int m, int k, int n) {
 
 }  // namespace
 
-// CTAs per cluster of the single-problem slice GEMM (1, or 2 = a CTA pair
+// CTAs per cluster of the single-problem residue GEMM (1, or 2 = a CTA pair
 // computing one 256-row tile with cta_group::2 MMAs, each CTA loading its own
 // half of the operands): PHPC_CLUSTER, else the table's choice where pairs
 // suit the shape, else 1.
 int default_cluster(int m, int k, int n) {
-  const char* env = getenv("PHPC_CLUSTER");
-  if (env && (atoi(env) == 1 || atoi(env) == 2)) return atoi(env);
+  if (const int c = env_cluster()) return c;
   if (const TuneEntry* e = lookup(m, k, n))
     if (e->cluster == 2 && pairs_fit(m, k, n)) return 2;
   return 1;
@@ -316,8 +361,10 @@ extern "C" int phpc_tuning(int m, int k, int n, int* cfg) {
   using namespace phpc;
   if (!cfg || m < 0 || k < 0 || n < 0) return PHPC_ERR_ARG;
   const F32Tune f = default_f32(m, k, n);
-  const int v[10] = {default_moduli(m, k, n), default_slices(m, k, n), default_bn(m, k, n),
-                     default_group_rows(m, k, n), default_cluster(m, k, n), default_stages(m, k, n),
+  const int q = default_moduli(m, k, n);
+  const int v[10] = {q, default_slices(m, k, n), q ? default_bn(m, k, n) : digit_bn(m, k, n),
+                     default_group_rows(m, k, n), q ? default_cluster(m, k, n) : digit_cluster(m, k, n),
+                     default_stages(m, k, n),
                      f.bn, f.group_rows, f.stages, default_plain_stages(m, k, n)};
   for (int i = 0; i < 10; ++i) cfg[i] = v[i];
   return PHPC_OK;
