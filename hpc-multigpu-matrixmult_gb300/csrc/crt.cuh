@@ -363,43 +363,67 @@ __device__ __forceinline__ void crt_limbs_quad(const uint32_t (&w)[2][kCrtMaxMod
 // c + y 2^x for a reconstructed y, |y| <= M (1/2 - 1/32): y rounded once to
 // double (to nearest even), the sum rounded once.
 //
-// Up to 13 moduli |y| < 2^108.6: with V = floor(y / 2^52) (64 bits) and A its
-// low 52 bits, y = B 2^58 + A', B = V >> 6 (|B| < 2^51), 0 <= A' < 2^58. Both
-// halves become doubles through their bits: 2^58 + A' with A''s low 6 bits
-// folded into one sticky bit, and (B - 1) 2^58 by one exact subtraction of a
-// constant; their sum is y's one rounding (for |y| >= 2^60 half an ulp lies
-// above the sticky bit). |V| < 2^32 (a zero, a strong cancellation) is rare:
-// there V is exact in double and so is A. Three FP64 additions a value: 48
-// cycles of the SM's FP64 pipe a warp, below the 58 that a warp's 42 bytes an
-// element take at DRAM speed. The kernel: N = 4096 158 -> 130 us (5.4 TB/s),
-// 16384 2.8 -> 2.24 ms, 512-problem batch 1.81 -> 1.59 ms.
+// Up to 14 moduli y is cut in two, floor(y / 2^s) and the s bits below. Each
+// half becomes a double through its bits, the upper one by an exact subtraction
+// of a constant, and their sum is y's one rounding:
+//  - 8 to 12 moduli (|y| < 2^100.4): s = 52, V = floor(y / 2^52), |V| < 2^48.4;
+//    (V - 1) 2^52 and 2^52 + the lower half are exact.
+//  - 13 and 14 moduli (|y| < 2^108.6, 2^116.9): s = 52 + SH, B = floor(y / 2^s),
+//    |B| < 2^51; (B - 1) 2^s is exact, and 2^s + the lower half has its low SH
+//    bits folded into one sticky bit, which lies below half an ulp of y for
+//    |y| >= 2^(SH + 54). Values below 2^84 (a zero, a strong cancellation) are
+//    rare and take the first form.
+// Three FP64 additions a value: 48 cycles of the SM's FP64 pipe a warp, below
+// the 58 that a warp's 42 bytes an element take at DRAM speed with 13 moduli.
+// Comparing doubles or converting an int64 costs that pipe as much again, so a
+// zero is found by its bits (8 moduli: 142 us with r == 0.0).
+//
+// The kernel at N = 4096, y rounded in 128-bit integers (crt_add_i128) / so: 8
+// moduli 114 us, 116; 9 130, 117; 10 136, 119; 11 148, 124; 12 152, 130; 13 160,
+// 132; 14 173, 148. (13 at N = 16384 2.8 ms, 2.24; 512-problem batch 1.81, 1.59.)
+// With 15 moduli the integers are the faster ones (191 us against 203).
 template <int NMOD>
 __device__ __forceinline__ double crt_round_add(double c, const CrtWords& y, int x) {
-  if (NMOD <= 13) {
-    const uint64_t w0 = static_cast<uint64_t>(y.w[0]);
-    const int64_t V = static_cast<int64_t>(static_cast<uint64_t>(y.w[1]) + static_cast<uint64_t>(y.w[0] >> 52) +
-                                           (static_cast<uint64_t>(y.w[2]) << 52));
-    double r;
-    if (static_cast<uint32_t>(static_cast<int32_t>(V >> 32) + 1) <= 1u) {
-      const double a = __longlong_as_double(static_cast<long long>((w0 & ((1ull << 52) - 1)) | (0x433ull << 52))) - 0x1p52;
-      r = fma(static_cast<double>(V), 0x1p52, a);
-      if (r == 0.0) return c + 0.0;
+  if constexpr (NMOD <= 14) {
+    constexpr int SH = NMOD == 14 ? 14 : 6;
+    constexpr uint64_t kFold = (1ull << SH) - 1;
+    constexpr double kUnit = SH == 14 ? 0x1p66 : 0x1p58;  // 2^s
+    const uint64_t low = static_cast<uint64_t>(y.w[0]) & ((1ull << 52) - 1);
+    // y = low + 2^52 mid, with 14 moduli (where that mid passes 64 bits) + 2^104 w[2]
+    int64_t mid = y.w[1] + (y.w[0] >> 52), B;
+    bool small;
+    if (NMOD <= 13) {
+      mid += static_cast<int64_t>(static_cast<uint64_t>(y.w[2]) << 52);
+      B = mid >> SH;
+      small = static_cast<uint32_t>(static_cast<int32_t>(mid >> 32) + 1) <= 1u;
     } else {
-      const uint32_t h0 = static_cast<uint32_t>(w0 >> 32), l0 = static_cast<uint32_t>(w0);
-      const uint32_t lo = __funnelshift_r(l0, h0, 6) | ((l0 & 63u) != 0 ? 1u : 0u);
-      const uint32_t hi = ((h0 >> 6) & 0x3FFFu) | ((static_cast<uint32_t>(V) << 14) & 0xFC000u) | ((1023u + 58u) << 20);
-      const int64_t zb = (V >> 6) + static_cast<int64_t>((1023ull + 52 + 58) << 52 | 1ull << 51);
-      const double xb = __longlong_as_double(zb) - (0x1.8p52 + 1.0) * 0x1p58;  // (B - 1) 2^58
-      r = xb + __hiloint2double(static_cast<int>(hi), static_cast<int>(lo));
+      B = (mid >> SH) + static_cast<int64_t>(static_cast<uint64_t>(y.w[2]) << (52 - SH));
+      small = static_cast<uint64_t>(B + (1ll << (32 - SH))) < (2ull << (32 - SH));
+    }
+    double r;
+    if (NMOD <= 12 || small) {
+      const int64_t V =
+          NMOD <= 13 ? mid : static_cast<int64_t>(static_cast<uint64_t>(B) << SH | (static_cast<uint64_t>(mid) & kFold));
+      const int64_t top = V + static_cast<int64_t>((1023ull + 104) << 52 | 1ull << 51);
+      r = (__longlong_as_double(top) - (0x1.8p104 + 0x1p52)) +
+          __longlong_as_double(static_cast<long long>(low | (1023ull + 52) << 52));
+      if (__double2hiint(r) == 0) return c + 0.0;
+    } else {
+      const uint64_t bits =
+          (static_cast<uint64_t>(mid) & kFold) << (52 - SH) | low >> SH | ((low & kFold) != 0 ? 1 : 0);
+      const int64_t top = B + static_cast<int64_t>((1023ull + 104 + SH) << 52 | 1ull << 51);
+      r = (__longlong_as_double(top) - (0x1.8p52 + 1.0) * kUnit) +
+          __longlong_as_double(static_cast<long long>(bits | (1023ull + 52 + SH) << 52));
     }
     return crt_add_scaled(c, r, x);
+  } else {
+    // y modulo 2^128
+    const uint64_t b_lo = static_cast<uint64_t>(y.w[1]) << 52;
+    const uint64_t lo = static_cast<uint64_t>(y.w[0]) + b_lo;
+    const uint64_t hi = static_cast<uint64_t>(y.w[0] >> 63) + static_cast<uint64_t>(y.w[1] >> 12) +
+                        (static_cast<uint64_t>(y.w[2]) << 40) + (lo < b_lo ? 1 : 0);
+    return crt_add_i128(c, lo, hi, x);
   }
-  // y modulo 2^128
-  const uint64_t b_lo = static_cast<uint64_t>(y.w[1]) << 52;
-  const uint64_t lo = static_cast<uint64_t>(y.w[0]) + b_lo;
-  const uint64_t hi = static_cast<uint64_t>(y.w[0] >> 63) + static_cast<uint64_t>(y.w[1] >> 12) +
-                      (static_cast<uint64_t>(y.w[2]) << 40) + (lo < b_lo ? 1 : 0);
-  return crt_add_i128(c, lo, hi, x);
 }
 
 // *c += v * 2^(shift + e): the CRT result of one element applied to C

@@ -501,12 +501,15 @@ __device__ __forceinline__ void residue_col_block(const double* __restrict__ B, 
 // 128-byte run of each plane row and a warp's loads cover 4 columns of 8 rows.
 constexpr int kColBlockK = 64, kColBlockJ = 32;
 
-// Blocks of 128 threads per SM the CRT kernels are held to up to 13 moduli
-// (above, the compiler's choice, 5): they wait on their loads of the residue
-// planes, so warps in flight count for more than a few spilled registers. The
-// grouped kernel holds its problem's fields too (7 blocks: batch 6.88 ms, 8:
-// 7.07, no bound, 5 blocks: 7.17).
-constexpr int crt_min_blocks(int nmod, bool grouped) { return nmod > 13 ? 5 : grouped ? 7 : 8; }
+// Blocks of 128 threads per SM the CRT kernels are held to: they wait on their
+// loads of the residue planes, so warps in flight count for more than a few
+// spilled registers. 13 moduli: single call 8 (N = 4096 132 us; 9 blocks 150),
+// grouped, which holds its problem's fields too, 7 (batch 6.88 ms, 8: 7.07, no
+// bound, 5 blocks: 7.17). 8 to 12: 8 (8 moduli 116 us; 6 blocks 125, 10 119, 12
+// 144). 14: 7 (148 us; 5 175, 6 160, 8 157). 15: 5 (191 us; 4 210, 6 523).
+constexpr int crt_min_blocks(int nmod, bool grouped) {
+  return nmod > 14 ? 5 : nmod == 14 || grouped ? 7 : 8;
+}
 
 constexpr int kCrtCols = 4;  // consecutive columns per thread (one 8-byte load per residue plane)
 
