@@ -301,6 +301,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   uint64_t* uq_empty = uq_full + kTcUnitQ;  // [kTcUnitQ] MMA issuer and epilogue warps -> producer
   int2* uq_unit = reinterpret_cast<int2*>(uq_empty + kTcUnitQ);  // [kTcUnitQ] (unit, its K-steps)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(uq_unit + kTcUnitQ);
+  uint32_t* share_missing = tmem_slot + 1;  // KSPLIT: an epilogue warp gave up before it put its sums
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // Work units: 128 x BN tiles (CLUSTER = 1) or 256 x BN pair tiles (CLUSTER = 2).
@@ -329,6 +330,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       mbar_init(&uq_full[q], 1);
       mbar_init(&uq_empty[q], 1 + kTcEpiWarps);
     }
+    *share_missing = 0;
     fence_mbar_init();
   }
   if (!GROUPED) pdl_trigger();
@@ -841,7 +843,12 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     }
     if (MODE == kResidue && !KSPLIT && lane == 0) bulk_wait_all();  // the stores have left shared memory
     if (KSPLIT) {
-      cluster_sync();  // every CTA's sums are in its shared memory
+      if (!ok && lane == 0) *share_missing = 1;
+      cluster_sync();  // every CTA's sums are in its shared memory, unless it gave up
+      // A unit with a share missing (a bounded wait expired, the status says so)
+      // is left alone, as an unsplit one is: all CTAs of the cluster see the same.
+      const uint32_t missing =
+          ld_shared_cluster_u32(mapa_shared(smem_u32(share_missing), min(lane, args.ksplit - 1)));
       int t, p0;
       tc_unit(unit0, ntiles, split, t, p0);
       TcJob job;
@@ -884,6 +891,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                                      : make_float4(sum[u].x + v[q][u].x, sum[u].y + v[q][u].y, sum[u].z + v[q][u].z,
                                                    sum[u].w + v[q][u].w);
         }
+        if (__any_sync(0xffffffffu, missing != 0)) break;
 #pragma unroll
         for (int u = 0; u < kBatch; ++u) {
           const int i = i0 + u * kTcEpiWarps * 32, r = r0 + i / kChunks, col = job.rn * BN + 4 * (i % kChunks);
