@@ -362,7 +362,7 @@ extern "C" int phpc_tuning(int m, int k, int n, int* cfg) {
   if (!cfg || m < 0 || k < 0 || n < 0) return PHPC_ERR_ARG;
   const F32Tune f = default_f32(m, k, n);
   const int q = default_moduli(m, k, n);
-  const int v[10] = {q, default_slices(m, k, n), q ? default_bn(m, k, n) : digit_bn(m, k, n),
+  const int v[10] = {q, default_slices(m, k, n), q ? modular_bn(m, k, n, q) : digit_bn(m, k, n),
                      default_group_rows(m, k, n), q ? default_cluster(m, k, n) : digit_cluster(m, k, n),
                      default_stages(m, k, n),
                      f.bn, f.group_rows, f.stages, default_plain_stages(m, k, n)};

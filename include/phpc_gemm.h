@@ -258,11 +258,15 @@ int phpc_default_slices(int m, int k, int n);
  * the fewest moduli giving a grid of at least 51 bits). */
 int phpc_default_moduli(int m, int k, int n);
 
-/* The configuration the library uses for an m x k x n problem (tuning table,
- * environment overrides, built-in defaults; no reference counterpart), in
- * cfg[10]: FP64-accurate GEMM moduli (0 = digit scheme), slices, tile width,
- * raster height, CTAs per cluster, ring stages (0 = deepest that fits); 3xBF16
- * GEMM tile width, raster height, stages; plain FP64 GEMM ring stages. */
+/* The configuration the device calls use for an m x k x n problem on the
+ * current device (environment overrides, the tuning table, the rules that
+ * narrow its tiles for few of them, built-in defaults; no reference
+ * counterpart), in cfg[10]: FP64-accurate GEMM moduli (0 = digit scheme; the
+ * next entries are that scheme's), slices, tile width, raster height, CTAs per
+ * cluster, ring stages (0 = deepest that fits); 3xBF16 GEMM tile width, raster
+ * height, stages; plain FP64 GEMM ring stages. phpc_gemm_cublas and the panels
+ * on the modular scheme keep the table's tile width where the device calls
+ * narrow it. */
 int phpc_tuning(int m, int k, int n, int *cfg);
 
 /* ------------------------------------------------------------------ utils */
