@@ -163,11 +163,11 @@ int f32_ksplit(int m, int n, int steps, const DeviceInfo* dev) {
 // The same for a residue GEMM whose (tile, modulus) units leave SMs idle. A
 // K-step takes 0.33 us whatever the tile width (48 KB, or 32, at an SM's share
 // of the L2 rate), and the shares' exchange through shared memory 4-6 us, so it
-// pays from 40 steps (K > 2496). GEMM alone, unsplit / split: 128 x 8192 x 128
-// 45.3 us, 20.9 with 8; 256 x 8192 x 256 53.8, 29.4 with 4; 336 x 4001 x 72
-// 26.8, 20.6 with 3; 235 x 3167 x 169 22.7, 18.6 with 3; 569 x 3453 x 178 24.7,
-// 22.7 with 2; but 128 x 2048 x 128 16.5, 16.9 with 8, and 640 x 1500 x 256
-// 14.8, 18.5 with 2. The residues are exact, so the bits do not depend on it.
+// pays from 40 steps (K > 2496). GEMM alone with 256-wide tiles, unsplit /
+// split: 128 x 8192 x 128 45.3 us, 20.9 with 8; 256 x 8192 x 256 53.8, 29.4 with
+// 4; 336 x 4001 x 72 26.8, 20.6 with 3; 235 x 3167 x 169 22.7, 18.6 with 3; 569 x
+// 3453 x 178 24.7, 22.7 with 2; but 128 x 2048 x 128 16.5, 16.9 with 8, and 640 x
+// 1500 x 256 14.8, 18.5 with 2. The residues are exact, so the bits do not depend on it.
 // PHPC_RESIDUE_KSPLIT = 1..8 forces it.
 template <int BN>
 int residue_ksplit(int64_t units, int steps, const DeviceInfo* dev) {
@@ -180,6 +180,24 @@ int residue_ksplit(int64_t units, int steps, const DeviceInfo* dev) {
 }
 
 }  // namespace
+
+// Whether a residue GEMM whose 128-wide units all run at once does better with
+// 256-wide ones because these, half as many, are split along K at least three
+// times as finely and each share is 30 K-steps shorter or more. Whole calls, 128 /
+// 256: 8 moduli, 569 x K x 178 (80 units unsplit, 40 by 3): K = 2600 49.5 us, 49.4;
+// 3453 55.8, 52.5; 4500 68.2, 61.4; 6000 85.0, 76.8; 13 moduli, 100 x K x 700 (78,
+// 39 by 3): 51.4, 54.1; 61.8, 60.0; 74.2, 72.4; 95.6, 92.5. With twice as fine a
+// split they come out even: 13 moduli, 569 x K x 178 (130, 65 by 2) 53.0, 55.6;
+// 63.0, 61.9; 75.5, 75.9; 92.6, 92.6; 250 x K x 500 (104, 52 by 2) 52.4, 55.7;
+// 62.7, 63.0; 73.9, 76.5; 91.2, 94.0.
+bool residue_wide_split(int m, int k, int n, int moduli, const DeviceInfo* dev) {
+  const int steps = ceil_div(k, kTcBK);
+  const int64_t rows = (int64_t)ceil_div(m, kTcBM) * moduli;
+  const int wide = residue_ksplit<256>(rows * ceil_div(n, 256), steps, dev);
+  if (wide < 3) return false;
+  const int narrow = residue_ksplit<128>(rows * ceil_div(n, 128), steps, dev);
+  return wide >= 3 * narrow && steps / narrow - steps / wide >= 30;
+}
 
 // Whether the 3xBF16 GEMM splits K and all its 128-wide tiles would run at
 // once with that split too.

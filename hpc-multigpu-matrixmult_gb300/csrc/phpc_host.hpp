@@ -165,6 +165,7 @@ struct F32Tune {
   int bn, group_rows, stages;
 };
 F32Tune default_f32(int m, int k, int n);
+bool residue_wide_split(int m, int k, int n, int moduli, const DeviceInfo* dev);
 bool f32_narrow_split(int m, int k, int n, const DeviceInfo* dev);
 constexpr int kF32SplitSteps = 48;  // K-steps (six products of each 64 of K) from which the 3xBF16 GEMM splits K
 // Stages of the grouped GEMM (the "grouped" entry's fifth field; 0 = deepest).

@@ -206,13 +206,17 @@ int digit_cluster(int m, int k, int n) {
 // 86 x 1343 x 615 33.5 us, 31.4; 235 x 3167 x 169 48.0, 45.6; 124 x 2991 x 1317
 // (143 units) 89.9, 87.1; 336 x 4001 x 72 50.4, 47.1; 8000 x 1000 x 100 143, 137;
 // N = 256 17.8, 16.4 as a graph. With more units than SMs the wide tile's fewer
-// operand bytes count: GEMM of 664 x 1420 x 668 22.8, 35.0. Exact either way.
+// operand bytes count: GEMM of 664 x 1420 x 668 22.8, 35.0; so does its K split
+// where that is much the finer one (residue_wide_split). Exact either way.
 int modular_bn(int m, int k, int n, int moduli) {
   const int bn = default_bn(m, k, n);
   if (bn == 128 || getenv("PHPC_OZAKI_BN")) return bn;
   if (n <= 128) return 128;
   const DeviceInfo* dev = current_device();
-  return dev && (int64_t)ceil_div(m, 128) * ceil_div(n, 128) * moduli <= dev->sm_count ? 128 : bn;
+  return dev && (int64_t)ceil_div(m, 128) * ceil_div(n, 128) * moduli <= dev->sm_count &&
+                 !residue_wide_split(m, k, n, moduli, dev)
+             ? 128
+             : bn;
 }
 
 namespace {
