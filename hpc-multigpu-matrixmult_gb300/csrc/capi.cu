@@ -241,8 +241,8 @@ int host_gemm(Method method, const double* a, int lda, const double* b, int ldb,
 // concurrent tiles, SMs / cluster size), at most 8 panels; problems too small
 // for two such panels use four panels of whole tile rows (or one below 2048
 // rows).
-int panel_rows(int m, int k, int n, int sms) {
-  const int bn = default_bn(m, k, n), cl = default_cluster(m, k, n);
+int panel_rows(int m, int k, int n, int nmod, int sms) {
+  const int bn = default_bn(m, k, n), cl = default_cluster(m, k, n, nmod);
   const int64_t tn = ceil_div(n, bn), units = std::max(1, sms / cl);
   const int64_t unit_rows = units / std::gcd(units, tn) * 128 * cl;
   int64_t pr;
@@ -290,10 +290,10 @@ int host_gemm_modular(const double* a, int lda, const double* b, int ldb, double
   pin(pb, b, ((size_t)(k - 1) * ldb + n) * sizeof(double));
   pin(pc, c, ((size_t)(m - 1) * ldc + n) * sizeof(double));
 
-  const int pr = panel_rows(m, k, n, dev->sm_count);
+  const int pr = panel_rows(m, k, n, nmod, dev->sm_count);
   const int np = ceil_div(m, pr);
   const int bn = default_bn(m, k, n);
-  const int nbp = np > 1 ? b_panels(pr, n, bn, default_cluster(m, k, n), dev->sm_count) : 1;
+  const int nbp = np > 1 ? b_panels(pr, n, bn, default_cluster(m, k, n, nmod), dev->sm_count) : 1;
   const int bcols = nbp == 1 ? n : ceil_div(ceil_div(n, nbp), bn) * bn;
   const int nbpanels = ceil_div(n, bcols);
   const size_t ws_bytes = ozaki2_workspace_bytes(m, k, n, nmod);

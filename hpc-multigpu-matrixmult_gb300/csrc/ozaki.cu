@@ -227,7 +227,9 @@ int launch_tc_slice_gemm(const void* planesA, const void* planesB, int nplanesA,
             ck = opt.cfg_k > 0 ? opt.cfg_k : k;
   // the 3xBF16 GEMM has its own table entries ("f32") and runs on single CTAs
   const F32Tune f32 = MODE == kF32 ? default_f32(cm, ck, cn) : F32Tune{};
-  const int cluster = MODE == kF32 ? 1 : MODE == kOzaki ? digit_cluster(cm, ck, cn) : default_cluster(cm, ck, cn);
+  const int cluster = MODE == kF32     ? 1
+                      : MODE == kOzaki ? digit_cluster(cm, ck, cn)
+                                       : default_cluster(cm, ck, cn, pairs.n);
   const uint32_t bB[3] = {kTcBK, (uint32_t)(BN / cluster), 1};  // with a 2-CTA cluster each CTA loads half of B
   if (!encode_tiled(&tmA, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, planesA, dA, sA, bA, CU_TENSOR_MAP_SWIZZLE_128B) ||
       !encode_tiled(&tmB, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, planesB, dB, sB, bB, CU_TENSOR_MAP_SWIZZLE_128B))

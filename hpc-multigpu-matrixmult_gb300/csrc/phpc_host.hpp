@@ -153,7 +153,7 @@ int digit_cluster(int m, int k, int n);  // and CTAs per cluster
 int modular_bn(int m, int k, int n, int moduli);
 int default_grouped_bn(const phpc_gemm_problem* problems, int count);
 int default_group_rows(int m, int k, int n);
-int default_cluster(int m, int k, int n);
+int default_cluster(int m, int k, int n, int moduli);
 // Pipeline depths: K-stages of the tcgen05 engine's shared-memory ring for
 // the FP64-accurate GEMMs (0 = the deepest ring that fits), of the 3xBF16
 // FP32 GEMM, and of the plain FP64 GEMM (2 .. 6).

@@ -221,22 +221,28 @@ int modular_bn(int m, int k, int n, int moduli) {
 
 namespace {
 
-// Whether CTA pairs suit the shape where the table has them. A pair stages 32
-// KB a K-step and SM against 48, but its units cost more to start and to drain:
-//  - fewer than 80 K-steps an SM (residue GEMM, 13 moduli): N = 1024 25.5 us
-//    single, 29.0 in pairs; 1024 x 2048 x 1024 49.1, 47.4; 2048 x 512 x 2048
-//    51.9, 48.2;
+// Whether CTA pairs suit a residue GEMM where the table has them. A pair stages
+// 32 KB a K-step and SM against 48, but its units cost more to start and to
+// drain (GEMM alone in us, single / pairs, 13 moduli unless named):
+//  - fewer than 80 K-steps an SM: N = 1024 (44 an SM) 25.4, 29.1; 1024 x 1536 x
+//    1024 (66) 39.1, 39.2; 1024 x 2048 x 1024 (88) 47.5, 47.2; 2048 x 512 x 2048
+//    (88) 52.5, 48.2; 8 moduli, 1024 x 2048 x 1024 (54) 30.9, 33.5; 1500^3 (91)
+//    47.4, 47.2; 10 moduli, 1536 x 1500 x 1024 (76) 47.2, 47.3; 15, N = 1024 (51)
+//    33.7, 37.0;
 //  - a last accumulator chunk (of 8 K-steps) that is half empty or emptier, or
 //    a single short one, leaves the MMAs waiting for the drain of the pair's
 //    other chunk: 4096 x K x 4096 with K = 256 110, 148; 384 144, 145; 512
 //    171, 156; 520 208, 235; 700 227, 244; 830 258, 256; 1000 318, 285; 1100
 //    344, 362; 2000 548, 526;
-//  - an odd number of tile rows pads the last pair: 1400 (11 rows) 63.9, 70.1;
-//    600 x 4096 x 2000 (5) 109, 121; 1537 x 1000 x 2311 (13) 86.5, 84.3.
-bool pairs_fit(int m, int k, int n) {
-  const int64_t rows = ceil_div(m, 128), steps = ceil_div(k, 64), units = (rows + 1) / 2 * ceil_div(n, 256) * 13;
+//  - an odd number of tile rows pads the last pair: 14 shapes of 5 to 11 rows
+//    from 0.93 to 1.17 of the single CTAs' time, 1.03 on average; 26 of 13 to
+//    27 rows 0.94 to 1.11, 0.99 on average.
+bool pairs_fit(int m, int k, int n, int moduli) {
+  const DeviceInfo* dev = current_device();
+  const int64_t pairs = dev ? dev->sm_count / 2 : 76;
+  const int64_t rows = ceil_div(m, 128), steps = ceil_div(k, 64), units = (rows + 1) / 2 * ceil_div(n, 256) * moduli;
   const bool full = steps % 8 == 0 || steps % 8 > 4 || steps > 32;
-  return full && steps >= 8 && units * steps >= 80 * 76 && (rows % 2 == 0 || rows > 12);
+  return full && steps >= 8 && units * steps >= 80 * pairs && (rows % 2 == 0 || rows > 12);
 }
 
 }  // namespace
@@ -245,10 +251,10 @@ bool pairs_fit(int m, int k, int n) {
 // computing one 256-row tile with cta_group::2 MMAs, each CTA loading its own
 // half of the operands): PHPC_CLUSTER, else the table's choice where pairs
 // suit the shape, else 1.
-int default_cluster(int m, int k, int n) {
+int default_cluster(int m, int k, int n, int moduli) {
   if (const int c = env_cluster()) return c;
   if (const TuneEntry* e = lookup(m, k, n))
-    if (e->cluster == 2 && pairs_fit(m, k, n)) return 2;
+    if (e->cluster == 2 && pairs_fit(m, k, n, moduli)) return 2;
   return 1;
 }
 
@@ -367,7 +373,7 @@ extern "C" int phpc_tuning(int m, int k, int n, int* cfg) {
   const F32Tune f = default_f32(m, k, n);
   const int q = default_moduli(m, k, n);
   const int v[10] = {q, default_slices(m, k, n), q ? modular_bn(m, k, n, q) : digit_bn(m, k, n),
-                     default_group_rows(m, k, n), q ? default_cluster(m, k, n) : digit_cluster(m, k, n),
+                     default_group_rows(m, k, n), q ? default_cluster(m, k, n, q) : digit_cluster(m, k, n),
                      default_stages(m, k, n),
                      f.bn, f.group_rows, f.stages, default_plain_stages(m, k, n)};
   for (int i = 0; i < 10; ++i) cfg[i] = v[i];
