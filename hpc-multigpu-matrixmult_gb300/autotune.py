@@ -20,6 +20,10 @@ stages on the rectangular workload (M = 32768, N = 8192, K = 4096, FP32
 normal(0, 1), error against the FP64 product on sampled rows); for the plain
 FP64 GEMM the ring depth (2-6 stages) per size up to --plain-max-n.
 
+The sweep forces each choice through the environment, which also stands above
+the library's shape rules (csrc/tune.cu: narrower tiles for few of them, no CTA
+pairs where they do not fit); those apply on top of the table it writes.
+
 Writes tune_table.txt next to this file (copied into lib/ by the build, where
 the library reads it):
 

@@ -1,8 +1,12 @@
 // Scheme and tile selection for the FP64-accurate Ozaki GEMMs.
 //
 // Order of precedence for each choice: an environment variable, then the
-// tuning table written by the autotuner (PHPC_TUNE_TABLE, or tune_table.txt
-// next to the library), then a built-in default. Schemes: the modular one
+// tuning table (PHPC_TUNE_TABLE, or tune_table.txt next to the library;
+// autotune.py writes one), then a built-in default. The table is measured on
+// square problems; three rules go by the call's own shape and stand above it,
+// below the environment: modular_bn and f32_narrow take 128-wide tiles where the
+// table says 256, and pairs_fit refuses CTA pairs where the table has them.
+// Schemes: the modular one
 // (PHPC_MODULI = 8..15 residue GEMMs; built-in default: the fewest moduli
 // whose operand grid has at least 51 bits, Frobenius error about 2e-15 on
 // inputs whose exponents spread over 2^+-20 inside a row) or, with
@@ -72,8 +76,8 @@ std::string library_dir() {
 // slices bn [stages]" for grouped calls, "f32 max_mnk bn group_rows stages"
 // for the 3xBF16 GEMM, "plain max_mnk stages" for the plain FP64 GEMM and
 // "digits max_mnk bn cluster" where the digit GEMM's choice is not that of the
-// single-problem entry; '#' starts a comment line; the first entry whose max_mnk covers the
-// problem applies. Written by autotune.py.
+// single-problem entry; '#' starts a comment line; the first entry whose
+// max_mnk covers the problem applies.
 void load_table() {
   const char* env = getenv("PHPC_TUNE_TABLE");
   const std::string path = env ? std::string(env) : library_dir() + "/tune_table.txt";
