@@ -238,7 +238,7 @@ class Scheme:
             self.ws_bytes = phpc.ozaki2_workspace_bytes(n, n, n, moduli)
             self.gemms = moduli
             self.name = f"modular, {moduli} moduli"
-            self.launches = 7  # scan_rows, residue_rows, fill_int, scan_cols, residue_cols, tc GEMM, crt
+            self.launches = 7  # scan and residue split of A; scan, merge and split of B; tc GEMM, crt
         else:
             self.ws_bytes = phpc.ozaki_workspace_bytes(n, n, n, slices)
             self.gemms = ozaki_pairs(slices)

@@ -147,11 +147,12 @@ size_t phpc_ozaki2_workspace_bytes(int m, int k, int n, int moduli);
 int phpc_dgemm_ozaki2_dev(int m, int k, int n, const double *dA, int64_t lda, const double *dB, int64_t ldb,
                           double *dC, int64_t ldc, int moduli, void *workspace, size_t workspace_bytes, void *stream);
 
-/* The three phases of phpc_dgemm_ozaki2_dev (same workspace, same
- * workspace_bytes: a workspace below phpc_ozaki2_workspace_bytes that holds
- * planes with 16-byte aligned rows is accepted and laid out so): prepare = exponent and grid scans + residue split of A and B;
- * multiply = the residue GEMMs (one 16-bit residue per element and modulus, in the
- * workspace); reconstruct = CRT, rounding and
+/* The three phases of phpc_dgemm_ozaki2_dev, on the same workspace and with
+ * the same workspace_bytes (a workspace below phpc_ozaki2_workspace_bytes that
+ * holds planes with 16-byte aligned rows is accepted and laid out so):
+ * prepare = exponent and grid scans + residue split of A and B;
+ * multiply = the residue GEMMs (one 16-bit residue per element and modulus, in
+ * the workspace); reconstruct = CRT, rounding and
  * C += result * 2^(ea[i] - ba[i] + eb[j] - bb[j]). */
 int phpc_ozaki2_prepare_dev(int m, int k, int n, const double *dA, int64_t lda, const double *dB, int64_t ldb,
                             int moduli, void *workspace, size_t workspace_bytes, void *stream);
