@@ -25,7 +25,7 @@ __host__ __device__ constexpr int crt_digits(int n) {
 // sum_i t_i (M / m_i) = y (mod M), so the reconstruction needs no
 // per-modulus multiplication.
 
-// Constants of the reconstruction on FP32 limbs (crt_limbs_quad), the floats
+// Constants of the reconstruction on FP32 limbs (crt_limbs), the floats
 // in both lanes of a packed f32x2 operation.
 struct CrtLimbs {
   int np;                                 // digits of the largest M / m_i (5 .. 10)
@@ -229,46 +229,6 @@ __device__ __forceinline__ double crt_value(const uint32_t (&rr)[kCrtMaxModuli],
   return crt_round(l, T, fast, shift);
 }
 
-// c + y 2^x for a 128-bit two's complement integer y = (hi, lo), |y| < 2^127:
-// y is rounded once to double (to nearest even; the same rounding as
-// crt_round's) and the sum rounded once. The double y 2^x is assembled from
-// integer bits (sign, leading-one position, 53-bit mantissa), so the FP64
-// pipe, which is slow on this GPU, does one add per element.
-__device__ __forceinline__ double crt_add_i128(double c, uint64_t lo, uint64_t hi, int x) {
-  const uint64_t sign = hi & (1ull << 63);
-  if (sign) {  // magnitude
-    lo = ~lo + 1;
-    hi = ~hi + (lo == 0 ? 1 : 0);
-  }
-  if ((hi | lo) == 0) return c + 0.0;
-  uint64_t top, rest;
-  int e;  // position of the leading one
-  if (hi != 0) {
-    const int lz = __clzll(static_cast<long long>(hi));
-    top = lz ? (hi << lz) | (lo >> (64 - lz)) : hi;
-    rest = lz ? lo << lz : lo;
-    e = 127 - lz;
-  } else {
-    const int lz = __clzll(static_cast<long long>(lo));
-    top = lo << lz;
-    rest = 0;
-    e = 63 - lz;
-  }
-  uint64_t mant = top >> 11;  // 53 bits, leading one at bit 52
-  const uint64_t round_bit = (top >> 10) & 1, sticky = ((top & 0x3FF) | rest) != 0 ? 1 : 0;
-  mant += round_bit & (sticky | (mant & 1));
-  if (mant >> 53) {
-    mant >>= 1;
-    ++e;
-  }
-  const int E = e + 1023 + x;  // biased exponent of y 2^x
-  if (E >= 1 && E <= 2046)
-    return c + __longlong_as_double(static_cast<long long>(sign | (static_cast<uint64_t>(E) << 52) |
-                                                           (mant & ((1ull << 52) - 1))));
-  const double m = static_cast<double>(mant);  // outside the normal range: scale in double (rare)
-  return c + ldexp(sign ? -m : m, e - 52 + x);
-}
-
 // A reconstructed integer y = w[0] + w[1] 2^52 + w[2] 2^104, the words signed
 // and overlapping (|w[0]|, |w[1]| < 2^63).
 struct CrtWords {
@@ -281,10 +241,9 @@ __device__ __forceinline__ int64_t mad_wide(int a, int b, int64_t c) {
   return d;
 }
 
-// The one-step CRT of four adjacent elements on FP32 limbs: two pairs, each
-// pair in the two lanes of packed f32x2 operations, both pairs computed in
-// one pass over the moduli so that each modulus's constants are read once
-// for the four elements. w[p][i] holds the stored t_i of pair p for modulus i
+// The one-step CRT of 2 PAIRS adjacent elements on FP32 limbs, each pair in the
+// two lanes of packed f32x2 operations, all pairs computed in one pass over the
+// moduli so that each modulus's constants are read once. w[p][i] holds the stored t_i of pair p for modulus i
 // (BF16, its first element in the low 16 bits, the second in the high 16
 // bits). Valid when every result satisfies |y| / M <= 1/2 - 1/32
 // (CrtTable::fast); gives the y of crt_value, element e = 2 p + lane. Every
@@ -305,31 +264,31 @@ __device__ __forceinline__ int64_t mad_wide(int a, int b, int64_t c) {
 // element on the integer pipe, its limit; see crt_round_add for the rounding.)
 // NMOD = T.n, the number of moduli; NP = T.L.np = crt_digits(NMOD), the
 // number of digits of the largest M / m_i.
-template <int NMOD>
-__device__ __forceinline__ void crt_limbs_quad(const uint32_t (&w)[2][kCrtMaxModuli], const CrtTable& T,
-                                               CrtWords (&out)[4]) {
+template <int NMOD, int PAIRS>
+__device__ __forceinline__ void crt_limbs(const uint32_t (&w)[PAIRS][kCrtMaxModuli], const CrtTable& T,
+                                          CrtWords (&out)[2 * PAIRS]) {
   constexpr int NP = crt_digits(NMOD);
   const float2 kRound = make_float2(12582912.0f, 12582912.0f), kUnround = make_float2(-12582912.0f, -12582912.0f);
-  float2 S[2][NP];
+  float2 S[PAIRS][NP];
 #pragma unroll
-  for (int p = 0; p < 2; ++p)
+  for (int p = 0; p < PAIRS; ++p)
 #pragma unroll
     for (int j = 0; j < NP; ++j) S[p][j] = make_float2(0.0f, 0.0f);
 #pragma unroll
   for (int i = 0; i < NMOD; ++i) {
-    float2 t[2];
+    float2 t[PAIRS];
 #pragma unroll
-    for (int p = 0; p < 2; ++p)
+    for (int p = 0; p < PAIRS; ++p)
       t[p] = make_float2(__uint_as_float(w[p][i] << 16), __uint_as_float(w[p][i] & 0xFFFF0000u));
 #pragma unroll
     for (int j = 0; j < NP; ++j) {
       const float2 pij = T.L.P[i][j];
-      S[0][j] = __ffma2_rn(t[0], pij, S[0][j]);
-      S[1][j] = __ffma2_rn(t[1], pij, S[1][j]);
+#pragma unroll
+      for (int p = 0; p < PAIRS; ++p) S[p][j] = __ffma2_rn(t[p], pij, S[p][j]);
     }
   }
 #pragma unroll
-  for (int p = 0; p < 2; ++p) {
+  for (int p = 0; p < PAIRS; ++p) {
     float2 est = __fmul2_rn(S[p][NP - 1], T.L.cw[0]);
     est = __ffma2_rn(S[p][NP - 2], T.L.cw[1], est);
     est = __ffma2_rn(S[p][NP - 3], T.L.cw[2], est);
@@ -363,67 +322,57 @@ __device__ __forceinline__ void crt_limbs_quad(const uint32_t (&w)[2][kCrtMaxMod
 // c + y 2^x for a reconstructed y, |y| <= M (1/2 - 1/32): y rounded once to
 // double (to nearest even), the sum rounded once.
 //
-// Up to 14 moduli y is cut in two, floor(y / 2^s) and the s bits below. Each
-// half becomes a double through its bits, the upper one by an exact subtraction
-// of a constant, and their sum is y's one rounding:
+// y is cut in two, floor(y / 2^s) and the s bits below. Each half becomes a
+// double through its bits, the upper one by an exact subtraction of a constant,
+// and their sum is y's one rounding:
 //  - 8 to 12 moduli (|y| < 2^100.4): s = 52, V = floor(y / 2^52), |V| < 2^48.4;
 //    (V - 1) 2^52 and 2^52 + the lower half are exact.
-//  - 13 and 14 moduli (|y| < 2^108.6, 2^116.9): s = 52 + SH, B = floor(y / 2^s),
-//    |B| < 2^51; (B - 1) 2^s is exact, and 2^s + the lower half has its low SH
-//    bits folded into one sticky bit, which lies below half an ulp of y for
-//    |y| >= 2^(SH + 54). Values below 2^84 (a zero, a strong cancellation) are
-//    rare and take the first form.
+//  - 13 to 15 moduli (|y| < 2^108.6, 2^116.9, 2^125.1): s = 52 + SH, B =
+//    floor(y / 2^s), |B| < 2^51; (B - 1) 2^s is exact, and 2^s + the lower half
+//    has its low SH bits folded into one sticky bit, which lies below half an
+//    ulp of y for |y| >= 2^(SH + 54). Values below 2^84 (a zero, a strong
+//    cancellation) are rare and take the first form.
 // Three FP64 additions a value: 48 cycles of the SM's FP64 pipe a warp, below
 // the 58 that a warp's 42 bytes an element take at DRAM speed with 13 moduli.
 // Comparing doubles or converting an int64 costs that pipe as much again, so a
 // zero is found by its bits (8 moduli: 142 us with r == 0.0).
 //
-// The kernel at N = 4096, y rounded in 128-bit integers (crt_add_i128) / so: 8
-// moduli 114 us, 116; 9 130, 117; 10 136, 119; 11 148, 124; 12 152, 130; 13 160,
-// 132; 14 173, 148. (13 at N = 16384 2.8 ms, 2.24; 512-problem batch 1.81, 1.59.)
-// With 15 moduli the integers are the faster ones (191 us against 203).
+// The kernel at N = 4096, digits assembled and rounded in 128-bit integers /
+// so: 8 moduli 114 us, 116; 9 130, 117; 10 136, 119; 11 148, 124; 12 152, 130; 13
+// 160, 132; 14 173, 148; 15 178, 166. (13 at N = 16384 2.8 ms, 2.24; 512-problem
+// batch 1.81, 1.59.)
 template <int NMOD>
 __device__ __forceinline__ double crt_round_add(double c, const CrtWords& y, int x) {
-  if constexpr (NMOD <= 14) {
-    constexpr int SH = NMOD == 14 ? 14 : 6;
-    constexpr uint64_t kFold = (1ull << SH) - 1;
-    constexpr double kUnit = SH == 14 ? 0x1p66 : 0x1p58;  // 2^s
-    const uint64_t low = static_cast<uint64_t>(y.w[0]) & ((1ull << 52) - 1);
-    // y = low + 2^52 mid, with 14 moduli (where that mid passes 64 bits) + 2^104 w[2]
-    int64_t mid = y.w[1] + (y.w[0] >> 52), B;
-    bool small;
-    if (NMOD <= 13) {
-      mid += static_cast<int64_t>(static_cast<uint64_t>(y.w[2]) << 52);
-      B = mid >> SH;
-      small = static_cast<uint32_t>(static_cast<int32_t>(mid >> 32) + 1) <= 1u;
-    } else {
-      B = (mid >> SH) + static_cast<int64_t>(static_cast<uint64_t>(y.w[2]) << (52 - SH));
-      small = static_cast<uint64_t>(B + (1ll << (32 - SH))) < (2ull << (32 - SH));
-    }
-    double r;
-    if (NMOD <= 12 || small) {
-      const int64_t V =
-          NMOD <= 13 ? mid : static_cast<int64_t>(static_cast<uint64_t>(B) << SH | (static_cast<uint64_t>(mid) & kFold));
-      const int64_t top = V + static_cast<int64_t>((1023ull + 104) << 52 | 1ull << 51);
-      r = (__longlong_as_double(top) - (0x1.8p104 + 0x1p52)) +
-          __longlong_as_double(static_cast<long long>(low | (1023ull + 52) << 52));
-      if (__double2hiint(r) == 0) return c + 0.0;
-    } else {
-      const uint64_t bits =
-          (static_cast<uint64_t>(mid) & kFold) << (52 - SH) | low >> SH | ((low & kFold) != 0 ? 1 : 0);
-      const int64_t top = B + static_cast<int64_t>((1023ull + 104 + SH) << 52 | 1ull << 51);
-      r = (__longlong_as_double(top) - (0x1.8p52 + 1.0) * kUnit) +
-          __longlong_as_double(static_cast<long long>(bits | (1023ull + 52 + SH) << 52));
-    }
-    return crt_add_scaled(c, r, x);
+  constexpr int SH = NMOD == 15 ? 23 : NMOD == 14 ? 14 : 6;
+  constexpr uint64_t kFold = (1ull << SH) - 1;
+  constexpr double kUnit = SH == 23 ? 0x1p75 : SH == 14 ? 0x1p66 : 0x1p58;  // 2^s
+  const uint64_t low = static_cast<uint64_t>(y.w[0]) & ((1ull << 52) - 1);
+  // y = low + 2^52 mid, from 14 moduli (where that mid passes 64 bits) + 2^104 w[2]
+  int64_t mid = y.w[1] + (y.w[0] >> 52), B;
+  bool small;
+  if (NMOD <= 13) {
+    mid += static_cast<int64_t>(static_cast<uint64_t>(y.w[2]) << 52);
+    B = mid >> SH;
+    small = static_cast<uint32_t>(static_cast<int32_t>(mid >> 32) + 1) <= 1u;
   } else {
-    // y modulo 2^128
-    const uint64_t b_lo = static_cast<uint64_t>(y.w[1]) << 52;
-    const uint64_t lo = static_cast<uint64_t>(y.w[0]) + b_lo;
-    const uint64_t hi = static_cast<uint64_t>(y.w[0] >> 63) + static_cast<uint64_t>(y.w[1] >> 12) +
-                        (static_cast<uint64_t>(y.w[2]) << 40) + (lo < b_lo ? 1 : 0);
-    return crt_add_i128(c, lo, hi, x);
+    B = (mid >> SH) + static_cast<int64_t>(static_cast<uint64_t>(y.w[2]) << (52 - SH));
+    small = static_cast<uint64_t>(B + (1ll << (32 - SH))) < (2ull << (32 - SH));
   }
+  double r;
+  if (NMOD <= 12 || small) {
+    const int64_t V =
+        NMOD <= 13 ? mid : static_cast<int64_t>(static_cast<uint64_t>(B) << SH | (static_cast<uint64_t>(mid) & kFold));
+    const int64_t top = V + static_cast<int64_t>((1023ull + 104) << 52 | 1ull << 51);
+    r = (__longlong_as_double(top) - (0x1.8p104 + 0x1p52)) +
+        __longlong_as_double(static_cast<long long>(low | (1023ull + 52) << 52));
+    if (__double2hiint(r) == 0) return c + 0.0;
+  } else {
+    const uint64_t bits = (static_cast<uint64_t>(mid) & kFold) << (52 - SH) | low >> SH | ((low & kFold) != 0 ? 1 : 0);
+    const int64_t top = B + static_cast<int64_t>((1023ull + 104 + SH) << 52 | 1ull << 51);
+    r = (__longlong_as_double(top) - (0x1.8p52 + 1.0) * kUnit) +
+        __longlong_as_double(static_cast<long long>(bits | (1023ull + 52 + SH) << 52));
+  }
+  return crt_add_scaled(c, r, x);
 }
 
 // *c += v * 2^(shift + e): the CRT result of one element applied to C

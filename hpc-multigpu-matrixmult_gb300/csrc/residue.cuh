@@ -506,10 +506,8 @@ constexpr int kColBlockK = 64, kColBlockJ = 32;
 // spilled registers. 13 moduli: single call 8 (N = 4096 132 us; 9 blocks 150),
 // grouped, which holds its problem's fields too, 7 (batch 6.88 ms, 8: 7.07, no
 // bound, 5 blocks: 7.17). 8 to 12: 8 (8 moduli 116 us; 6 blocks 125, 10 119, 12
-// 144). 14: 7 (148 us; 5 175, 6 160, 8 157). 15: 5 (191 us; 4 210, 6 523).
-constexpr int crt_min_blocks(int nmod, bool grouped) {
-  return nmod > 14 ? 5 : nmod == 14 || grouped ? 7 : 8;
-}
+// 144). 14: 7 (148 us; 5 175, 6 160, 8 157). 15: 7 (166 us; 6 175).
+constexpr int crt_min_blocks(int nmod, bool grouped) { return nmod >= 14 || grouped ? 7 : 8; }
 
 constexpr int kCrtCols = 4;  // consecutive columns per thread (one 8-byte load per residue plane)
 
@@ -536,7 +534,7 @@ inline void with_crt_moduli(int n, F&& f) {
 // row's exponent less its grid width). Columns at or beyond ncols are left
 // alone.
 // NMOD = T.n (the kernels are instantiated per modulus count); with fast
-// set the four elements are reconstructed on FP32 limbs (crt_limbs_quad),
+// set the four elements are reconstructed on FP32 limbs (crt_limbs),
 // else by the 32-bit-limb integer path (crt_value).
 template <int NMOD>
 __device__ __forceinline__ void crt_cols(const uint16_t* __restrict__ rp, int64_t rplane, const CrtTable& T, int fast,
@@ -553,8 +551,32 @@ __device__ __forceinline__ void crt_cols(const uint16_t* __restrict__ rp, int64_
       w[0][i] = rw[i].x;
       w[1][i] = rw[i].y;
     }
+    if constexpr (NMOD == 15) {
+      // one pair after the other: both at once need 92 registers (5 blocks an SM,
+      // or spills), 191-209 us at N = 4096 against 166
+      double cv[kCrtCols];
+#pragma unroll
+      for (int c = 0; c < kCrtCols; ++c) cv[c] = c < ncols ? cp[c] : 0.0;
+#pragma unroll
+      for (int p = 0; p < 2; ++p) {
+        uint32_t wp[1][kCrtMaxModuli];
+#pragma unroll
+        for (int i = 0; i < kCrtMaxModuli; ++i) {
+          wp[0][i] = w[p][i];
+          if (p == 1 && i < NMOD) asm volatile("" : "+r"(wp[0][i])::"memory");  // not before the first pair's stores
+        }
+        CrtWords y[2];
+        crt_limbs<NMOD, 1>(wp, T, y);
+#pragma unroll
+        for (int l = 0; l < 2; ++l) {
+          const int c = 2 * p + l;
+          if (c < ncols) cp[c] = crt_round_add<NMOD>(cv[c], y[l], row_shift + max(ebp[c], -20000) - bbp[c]);
+        }
+      }
+      return;
+    }
     CrtWords y[kCrtCols];
-    crt_limbs_quad<NMOD>(w, T, y);
+    crt_limbs<NMOD, 2>(w, T, y);
     if (ncols == kCrtCols) {
       double cv[kCrtCols];
 #pragma unroll

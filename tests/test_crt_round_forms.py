@@ -1,4 +1,4 @@
-"""The CRT's rounding for 8 to 14 moduli (csrc/crt.cuh, crt_round_add), modelled
+"""The CRT's rounding for every modulus count (csrc/crt.cuh, crt_round_add), modelled
 in Python integers and doubles: the reconstructed integer, given as limbs of
 weight 2^(13 j), is cut into an upper and a lower half, each becomes a double
 through its bits, and their sum must be its one correct rounding (Python's int
@@ -13,7 +13,7 @@ from test_crt_round import bits, limbs_of, s64, words
 
 
 def rounded(q, limbs):
-    sh = 0 if q <= 12 else {13: 6, 14: 14}[q]
+    sh = 0 if q <= 12 else {13: 6, 14: 14, 15: 23}[q]
     fold = (1 << sh) - 1
     w0, w1, w2 = words(limbs)
     low, mid = w0 % 2**52, w1 + (w0 >> 52)
@@ -37,7 +37,7 @@ def rounded(q, limbs):
     return upper + lower
 
 
-@pytest.mark.parametrize("q", list(range(8, 15)))
+@pytest.mark.parametrize("q", list(range(8, 16)))
 def test_one_correct_rounding(q):
     T = CL.Table(q)
     bound = T.M * 15 // 32

@@ -1,4 +1,4 @@
-"""The CRT's arithmetic up to its 64-bit words (csrc/crt.cuh, crt_limbs_quad),
+"""The CRT's arithmetic up to its 64-bit words (csrc/crt.cuh, crt_limbs),
 modelled on the CPU for every modulus count: t stored as BF16, limb sums and
 quotient in FP32, limbs converted to integers and four of them gathered in a
 word. (crt_limb_model.py keeps the earlier form: t stored with a bias, carries
